@@ -451,7 +451,7 @@ int stage_convolution_t(gg_ctx* ctx) {
         a.tw_off = ctx->d_tw_off;
         a.gtab = ctx->d_gtab;
         a.g_off = ctx->d_g_off;
-        launch_conv_f64(a, stage_grid(ctx, ST_CONV), conv_f64_smem_bytes(ctx->side_max), ctx->stream);
+        launch_conv_f64(a, stage_grid(ctx, ST_CONV), ctx->side_max, ctx->stream);
         ctx->launches += 3;
     } else {
         // two size classes in one step: sides up to kUmmaMaxSide on the tensor cores, larger
@@ -915,7 +915,7 @@ int supported_side(bool fp64) {
     for (;;) {
         const int m = n + 1;
         bool ok = redist_smem_bytes(m, fp64) <= lim && mc_slab_bytes(m) + 40 * 1024 <= lim;
-        if (fp64) ok = ok && conv_f64_smem_bytes(m) <= lim;
+        if (fp64) ok = ok && m <= kConvF64MaxSide;
         else ok = ok && 3 * (size_t)m * (m | 1) * 4 <= lim;
         if (!ok || m > 4096) return n;
         n = m;
@@ -1453,11 +1453,10 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     if (!d_in || !d_out || !sides || !offs || n_boxes < 1 || domain_size < 1) return GG_ERR_INVALID;
     int nmax = 0;
     for (int b = 0; b < n_boxes; b++) nmax = std::max(nmax, (int)sides[b]);
-    int dev = 0, sms = 0, optin = 0;
+    int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    if (nmax < 1 || conv_f64_smem_bytes(nmax) > (size_t)optin) return GG_ERR_UNSUPPORTED;
+    if (nmax < 1 || nmax > kConvF64MaxSide) return GG_ERR_UNSUPPORTED;
     std::vector<double2> tw;
     std::vector<long long> tw_off(nmax + 2, 0), g_off(nmax + 2, 0);
     std::vector<double> gt;
@@ -1516,7 +1515,7 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     a.tw_off = d_tw_off;
     a.gtab = d_gt;
     a.g_off = d_g_off;
-    launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, conv_f64_smem_bytes(nmax), 0);
+    launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, nmax, 0);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     void* ptrs[] = {d_tw, d_gt, d_tw_off, d_g_off, d_spec, d_box, d_off, d_spec_off, d_toff};

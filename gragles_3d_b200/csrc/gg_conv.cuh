@@ -22,8 +22,10 @@ struct ConvArgs {
     const long long* g_off;
 };
 
-size_t conv_f64_smem_bytes(int nmax);
-int conv_f64_max_side(size_t smem_limit);
-void launch_conv_f64(const ConvArgs& a, int grid, size_t smem, cudaStream_t s);
+// Largest box side the FP64 convolution takes: a plane and two complex half-spectra of
+// it in 227 KB of shared memory.
+constexpr int kConvF64MaxSide = 97;
+// nmax: the largest side among the boxes of the tiles.
+void launch_conv_f64(const ConvArgs& a, int grid, int nmax, cudaStream_t s);
 
 }  // namespace gg

@@ -36,6 +36,7 @@ namespace {
 
 constexpr int kMaxBoxes = 256;
 constexpr int kMaxSide = 96;
+static_assert(kMaxSide <= gg::kConvF64MaxSide, "sides the convolution takes");
 constexpr long long kScratchComplex = 1LL << 21;  // 2 Mi complex doubles = 32 MiB
 constexpr int kMaxDevices = 64;
 
@@ -153,12 +154,9 @@ extern "C" int gg_convolve_boxes_f64_noalloc(const double* d_in, double* d_out, 
         spec_total += (long long)n * n * (n / 2 + 1);
     }
     if (spec_total > kScratchComplex) return GG_ERR_UNSUPPORTED;
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return GG_ERR_CUDA;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = gg::conv_f64_smem_bytes(nmax);
-    if (smem > (size_t)optin) return GG_ERR_UNSUPPORTED;
 
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceState& d = g_dev[dev];
@@ -202,7 +200,7 @@ extern "C" int gg_convolve_boxes_f64_noalloc(const double* d_in, double* d_out, 
     // an error left over from earlier, unrelated work is not this launch's: clear it
     // first (a sticky error has already failed the copies above)
     (void)cudaGetLastError();
-    gg::launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, smem, 0);
+    gg::launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, nmax, 0);
     if (cudaGetLastError() != cudaSuccess) return GG_ERR_CUDA;
     if (cudaDeviceSynchronize() != cudaSuccess) return GG_ERR_CUDA;
     return GG_OK;

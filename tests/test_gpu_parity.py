@@ -61,6 +61,20 @@ def test_convolution_kernel_bitexact(gpu, oracle):
         assert np.array_equal(g, want), f"side {b.shape[0]}: max diff {np.abs(g - want).max()}"
 
 
+@pytest.mark.parametrize("sides", [[1, 2, 3, 4], [7, 8, 9, 6, 15, 16, 17], [23, 24, 25, 39, 40, 41], [55, 56, 57, 40],
+                                   [63, 64, 31], [65, 66, 8], [97, 81, 3]])
+def test_convolution_kernel_bitexact_at_fragment_edges(gpu, oracle, sides):
+    """Sides around the matrix instruction's 8 x 8 x 4 fragments (lines, frequencies and chain
+    lengths with every remainder), around pass B's switch to two line buffers (above 64) and
+    up to the largest side, the large ones beside small ones; the chains' order makes the
+    result equal to the oracle's bit for bit."""
+    rng = np.random.default_rng(17)
+    boxes = [rng.uniform(-0.1, 0.1, (n, n, n)) for n in sides]
+    got = gpu.convolve_boxes_f64(boxes, 100, 0.2)
+    for b, g in zip(boxes, got):
+        assert np.array_equal(g, oracle.convolve_box(b, 100, 0.2)), f"side {b.shape[0]}"
+
+
 def test_mixed_convolution_kernel_accuracy(gpu, oracle):
     """The mixed path's convolution (tcgen05 with operands split into FP16 hi + lo, three MMAs per
     K-step, when all sides are <= 64; FP32 SIMT otherwise) against the FP64 specified DFT: FP32-level error, far below plain TF32's
