@@ -15,7 +15,7 @@
 //   2. compare: one CTA per tile loads every covering box's values over the tile
 //      into shared memory once and looks up, in each covering grain's position
 //      table (built once per step from its comparison list), the position of every
-//      other covering grain in its list.  Per voxel it keeps the kTop
+//      voxel's two largest in its list.  Per voxel it keeps the kTop
 //      largest values; every (grain, voxel) pair then picks the first candidate
 //      that is in that grain's list, resolving equal values by list position --
 //      falling back to a full scan of the tile's boxes whenever the kTop
@@ -39,13 +39,14 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kTV = kTX * kTY * kTZ;   // voxels per tile (64)
-constexpr int kTop = 4;                // candidates kept per voxel
+constexpr int kTop = 3;                // candidates kept per voxel
 constexpr int kParts = kThreads / kTV; // threads scanning the boxes of one voxel
 // row stride of the staged values: the kParts lanes of a voxel read kVS apart, which
 // puts the 32 lanes of a warp on 32 different banks
 constexpr int kVS = kTV + 8;
 static_assert(kTV % 32 == 0 && kThreads % kTV == 0, "a warp's lanes share one tile entry per pair sweep");
-static_assert(kThreads == kTV * kParts && kTop == 4 && (kParts & (kParts - 1)) == 0, "top-4 merge layout");
+static_assert(kThreads == kTV * kParts && (kParts & (kParts - 1)) == 0, "merge layout");
+static_assert(kTX == 8 && kTY == 4 && kTZ == 2, "an entry's coverage of a tile is two 32-bit masks, a byte per row");
 constexpr unsigned kNone = 0xFFFFFFFFu;
 constexpr unsigned short kNotListed = 0xFFFF;
 constexpr int kUCap = 32;              // candidate columns of the position matrix
@@ -218,58 +219,79 @@ __global__ void __launch_bounds__(1024) bin_scan_kernel(TileBins tb, int n_tiles
 // ---------------------------------------------------------------------------------
 // 3. the per-tile comparison
 // ---------------------------------------------------------------------------------
+// One grain box reaching the tile.  Element offsets are of the tile's first voxel (they may
+// point before the box; only covered voxels are touched): voxel (dx, dy, dz) of the tile
+// lies dz * nxy + dy * nx + dx further.
+struct alignas(16) Entry {
+    long long in, out, idn;     // field, output and IDLocal
+    int nx, nxy;                // strides of its box
+    unsigned cover[2];          // covered voxels of the tile, one bit each, per z
+    uint32_t id;
+    unsigned flags;             // kBoundary, kActive
+};
+constexpr unsigned kBoundary = 1;  // the box reaches the boundary grain's zone
+constexpr unsigned kActive = 2;    // the grain is compared (recalculateIDLocal leaves non-existing ones alone)
+static_assert(sizeof(Entry) == 48, "three 16-byte loads");
+
 template <typename T>
 struct TileSmem {
-    // entries (boxes reaching the tile)
-    uint32_t* id;
-    int* box;           // 6 per entry
-    long long* off;
-    int* bbox;          // 6 per entry: new bounding box contributions
-    long long* outoff;  // per entry: offset of its output box and IDLocal box
-    long long* idoff;
-    int* tsize;         // per entry: size of its position table
+    Entry* ent;
     T* val;             // [entry][voxel]
-    unsigned short* pos;// [entry a][entry b]: position of b in a's list, kNotListed, or kUnknown
     T* topv;            // [kTop][voxel]
-    unsigned char* topi;
-    int* ncand;         // covering entries with value > -1, per voxel
-    unsigned* umask;    // 8 words: entries among some voxel's kTop candidates
-    unsigned char* ulist;  // those entries, ascending
-    unsigned char* ucol;   // per entry: its column of pos (the first kUCap of ulist), 0xFF: none
+    T* bthr;            // per voxel: the boundary distance's value wins over any neighbour value below this,
+    T* bset;            //   and is this
+    unsigned (*pmask)[2];  // per entry: voxels whose result is >= 0
+    int* tsize;         // per entry: size of its position table
+    unsigned* umask;    // 8 words: entries among some voxel's two largest
     int* nu;            // their count
-    unsigned char* bnd;    // per entry: its box reaches the boundary grain's zone
-    unsigned char* deep;   // per voxel: at least gb from every face of that zone
+    unsigned short* pos;// [entry a][column of b]: position of b in a's list, or kNotListed
+    unsigned char* ulist;  // column -> entry
+    unsigned char* ucol;   // entry -> column of pos (the first kUCap of ulist), 0xFF: none
+    unsigned char* topi;   // [kTop][voxel]
+    unsigned char* bunk;   // per voxel: no branch of the reference assigns its boundary distance
 };
+
+template <typename T>
+__host__ __device__ constexpr size_t tile_smem_bytes(int mcap) {
+    return (sizeof(Entry) + sizeof(T) * kVS + 8 + 4 + 2 * kUCap) * (size_t)mcap + sizeof(T) * kTV * (kTop + 2) + 48 + 512 +
+           kTV * (kTop + 1) + 64;
+}
 
 template <typename T>
 __device__ TileSmem<T> carve(unsigned char* base, int mcap) {
     TileSmem<T> s;
     unsigned char* p = base;
-    s.off = reinterpret_cast<long long*>(p); p += 8 * mcap;
-    s.outoff = reinterpret_cast<long long*>(p); p += 8 * mcap;
-    s.idoff = reinterpret_cast<long long*>(p); p += 8 * mcap;
+    s.ent = reinterpret_cast<Entry*>(p); p += sizeof(Entry) * mcap;
     s.val = reinterpret_cast<T*>(p); p += sizeof(T) * (size_t)mcap * kVS;
     s.topv = reinterpret_cast<T*>(p); p += sizeof(T) * kTV * kTop;
-    s.id = reinterpret_cast<uint32_t*>(p); p += 4 * mcap;
-    s.box = reinterpret_cast<int*>(p); p += 24 * mcap;
-    s.bbox = reinterpret_cast<int*>(p); p += 24 * mcap;
+    s.bthr = reinterpret_cast<T*>(p); p += sizeof(T) * kTV;
+    s.bset = reinterpret_cast<T*>(p); p += sizeof(T) * kTV;
+    s.pmask = reinterpret_cast<unsigned (*)[2]>(p); p += 8 * mcap;
     s.tsize = reinterpret_cast<int*>(p); p += 4 * mcap;
-    s.ncand = reinterpret_cast<int*>(p); p += 4 * kTV;
     s.umask = reinterpret_cast<unsigned*>(p); p += 4 * 8;
     s.nu = reinterpret_cast<int*>(p); p += 16;
     s.pos = reinterpret_cast<unsigned short*>(p); p += 2 * (size_t)mcap * kUCap;
     s.ulist = p; p += 256;
     s.ucol = p; p += 256;
     s.topi = p; p += kTV * kTop;
-    s.deep = p; p += kTV;
-    s.bnd = p;
+    s.bunk = p;
     return s;
 }
 
-// |in| < lim, lim in FP64, as (double)fabs(in) < lim: for FP32 values against the FP32
-// bound rounded up (a float is below a double exactly when it is below that bound).
-__device__ __forceinline__ bool in_band(double in, double lim) { return fabs(in) < lim; }
-__device__ __forceinline__ bool in_band(float in, double lim) { return fabsf(in) < __double2float_ru(lim); }
+// Bits lo .. hi - 1 of an n-bit row.
+__device__ __forceinline__ unsigned span_bits(int lo, int hi, int n) {
+    lo = max(lo, 0);
+    hi = min(hi, n);
+    return hi > lo ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) : 0u;
+}
+
+// The least T that is not below d: v < d, d in FP64, exactly when v is below it.
+template <typename T>
+__device__ __forceinline__ T not_below(double d);
+template <>
+__device__ __forceinline__ double not_below<double>(double d) { return d; }
+template <>
+__device__ __forceinline__ float not_below<float>(double d) { return __double2float_ru(d); }
 
 template <typename T>
 __device__ __forceinline__ T neg_inf();
@@ -278,19 +300,19 @@ __device__ __forceinline__ double neg_inf<double>() { return -CUDART_INF; }
 template <>
 __device__ __forceinline__ float neg_inf<float>() { return -CUDART_INF_F; }
 
-// Keep the kTop largest values seen so far in descending order (registers only).
+// Keep the kTop largest values seen so far in descending order, without branches.
 template <typename T>
 __device__ __forceinline__ void top_insert(T (&tv)[kTop], int (&ti)[kTop], T w, int e) {
-    if (!(w > tv[kTop - 1])) return;
-    tv[kTop - 1] = w;
-    ti[kTop - 1] = e;
+    bool above[kTop];
+#pragma unroll
+    for (int k = 0; k < kTop; k++) above[k] = w > tv[k];
 #pragma unroll
     for (int k = kTop - 1; k > 0; k--) {
-        if (tv[k] > tv[k - 1]) {
-            const T t = tv[k]; tv[k] = tv[k - 1]; tv[k - 1] = t;
-            const int u = ti[k]; ti[k] = ti[k - 1]; ti[k - 1] = u;
-        }
+        tv[k] = above[k - 1] ? tv[k - 1] : (above[k] ? w : tv[k]);
+        ti[k] = above[k - 1] ? ti[k - 1] : (above[k] ? e : ti[k]);
     }
+    tv[0] = above[0] ? w : tv[0];
+    ti[0] = above[0] ? e : ti[0];
 }
 
 __device__ __forceinline__ unsigned pos_home(uint32_t id, int size) { return (id * 2654435761u) & (unsigned)(size - 1); }
@@ -312,12 +334,89 @@ __device__ unsigned short list_position(const CompareArgs<T>& a, uint32_t ga, in
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 4) compare_kernel(CompareArgs<T> a) {
+__device__ __forceinline__ unsigned short pair_position(const TileSmem<T>& s, const CompareArgs<T>& a, int ea, int eb) {
+    const int col = s.ucol[eb];
+    return col != 0xFF ? s.pos[ea * kUCap + col] : list_position(a, s.ent[ea].id, s.tsize[ea], s.ent[eb].id);
+}
+
+// The neighbour entry that grain entry ea takes at voxel v, or -1: the largest listed value,
+// ties to the earliest position.  The general case: ties, unlisted candidates, no candidate.
+template <typename T>
+__device__ int decide_pair(const TileSmem<T>& s, const CompareArgs<T>& a, int ea, int v, int m) {
+    int best = -1;
+    unsigned short bpos = kNotListed;
+    T level = neg_inf<T>();
+    for (int k = 0; k < kTop; k++) {
+        const int eb = s.topi[k * kTV + v];
+        if (eb == 0xFF) return best;  // every covering candidate was among those examined
+        const T w = s.topv[k * kTV + v];
+        if (best >= 0 && !(w == level)) return best;
+        if (eb == ea) continue;
+        const unsigned short p = pair_position(s, a, ea, eb);
+        if (p == kNotListed) continue;
+        if (best < 0 || p < bpos) { best = eb; bpos = p; level = w; }
+    }
+    best = -1;  // full scan of the tile's boxes at this voxel
+    bpos = kNotListed;
+    for (int eb = 0; eb < m; eb++) {
+        if (eb == ea) continue;
+        const T w = s.val[eb * kVS + v];
+        if (!(w > T(-1))) continue;
+        if (best >= 0 && w < level) continue;
+        const unsigned short p = pair_position(s, a, ea, eb);
+        if (p == kNotListed) continue;
+        if (best < 0 || w > level || (w == level && p < bpos)) { best = eb; bpos = p; level = w; }
+    }
+    return best;
+}
+
+// The neighbour value and ID of a pair that its voxel's two largest values do not decide.  Not
+// inlined, and given the shared memory's base instead of the pointers into it: it is rare,
+// and the row loop keeps its registers.
+template <typename T>
+struct Neighbour {
+    T value;
+    uint32_t id;
+};
+template <typename T>
+__device__ __noinline__ Neighbour<T> slow_pair(unsigned char* smem, const CompareArgs<T>& a, int ea, int v, int m,
+                                               int y, int x, int z) {
+    const TileSmem<T> s = carve<T>(smem, a.mcap);
+    const int best = decide_pair(s, a, ea, v, m);
+    if (best >= 0) return Neighbour<T>{s.val[best * kVS + v], s.ent[best].id};
+    // no listed neighbour covers the voxel: value -1, IDLocal kept
+    const uint32_t g = s.ent[ea].id;
+    const Box A = load_box(a.in.box + 6 * g), Bold = load_box(a.idbox_old + 6 * g);
+    const long long f = A.at(y, x, z);
+    return Neighbour<T>{T(-1), f < Bold.count() ? a.id_old[a.idoff_old[g] + f] : 0u};
+}
+// The boundary distance where no branch assigns it at the voxel itself.
+template <typename T>
+__device__ __noinline__ double carried_dist(const CompareArgs<T>& a, uint32_t g, int y, int x, int z) {
+    return bc_dist(load_box(a.in.box + 6 * g), y, x, z, a.geo.M, a.geo.gb);
+}
+
+// One CTA per tile.  Bound by instruction issue: a tile of 64 voxels has ~50 boxes, so ~100
+// (box, 32 voxels) rows are staged, searched and written.  What a row needs is therefore
+// prepared once per box (one record with the three offsets, the strides and the covered
+// voxels as bit masks) or once per voxel and held in its thread's registers, whose voxel
+// stays the same over the boxes (candidates, their IDs, the boundary distance, which does
+// not depend on the box); the positive voxels of a row are one ballot, turned into the box's
+// extents at the end.  Per (box, voxel) pair this had been a walk over four candidates with
+// the boundary distance in FP64: 14.4 -> 8.3 ms for 820 M pairs (256^3 / 20,000 grains, FP32
+// storage), 2.75 -> 1.57 ms for 90 M (128^3 / 2,000, FP64); issue slots 61% busy, the ALU
+// pipe 59%.  Two voxels a lane (one row of both z) spill registers and took 9.1 ms.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 4) compare_kernel(const __grid_constant__ CompareArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileSmem<T> s = carve<T>(smem_raw, a.mcap);
     const TileBins& tb = a.bins;
     const int n_tiles = tb.ntx * tb.nty * tb.ntz;
     const T NEG = neg_inf<T>();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // this thread's voxel of the tile in the row loops (staging: half 0)
+    const int dx = lane & 7, dy = lane >> 3;
+    const T lim = not_below<T>(0.7 * a.geo.delta);
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
         const int e0 = tb.off[t], m = tb.off[t + 1] - e0;
         if (m == 0) continue;
@@ -327,136 +426,116 @@ __global__ void __launch_bounds__(kThreads, 4) compare_kernel(CompareArgs<T> a) 
         }
         const int tx = t % tb.ntx, ty = (t / tb.ntx) % tb.nty, tz = t / (tb.ntx * tb.nty);
         const int X0 = tx * kTX, Y0 = ty * kTY, Z0 = tz * kTZ;
-        // entries
-        for (int e = threadIdx.x; e < m; e += blockDim.x) {
+        for (int e = threadIdx.x; e < m; e += kThreads) {
             const uint32_t g = tb.entries[e0 + e];
-            s.id[e] = g;
-            const int* bb = a.in.box + 6 * g;
-#pragma unroll
-            for (int q = 0; q < 6; q++) s.box[6 * e + q] = bb[q];
-            s.off[e] = a.in.off[g];
-            s.outoff[e] = a.out.off[g];
-            s.idoff[e] = a.idoff_new[g];
+            const Box B = load_box(a.in.box + 6 * g);
+            Entry r;
+            r.nx = B.nx();
+            r.nxy = B.nx() * B.ny();
+            const long long at = (long long)(Z0 - B.z0) * r.nxy + (long long)(Y0 - B.y0) * r.nx + (X0 - B.x0);
+            r.in = a.in.off[g] + at;
+            r.out = a.out.off[g] + at;
+            r.idn = a.idoff_new[g] + at;
+            const unsigned ym = span_bits(B.y0 - Y0, B.y1 - Y0, kTY);
+            const unsigned rows = span_bits(B.x0 - X0, B.x1 - X0, kTX) *
+                                  ((ym & 1) | ((ym & 2) << 7) | ((ym & 4) << 14) | ((ym & 8) << 21));
+            r.cover[0] = B.z0 <= Z0 && Z0 < B.z1 ? rows : 0u;
+            r.cover[1] = B.z0 <= Z0 + 1 && Z0 + 1 < B.z1 ? rows : 0u;
+            r.id = g;
+            const bool inner = B.x0 > a.geo.gb && B.x1 < a.geo.M - a.geo.gb && B.y0 > a.geo.gb &&
+                               B.y1 < a.geo.M - a.geo.gb && B.z0 > a.geo.gb && B.z1 < a.geo.M - a.geo.gb;
+            r.flags = (inner ? 0u : kBoundary) | (a.set_comparison || a.exists[g] ? kActive : 0u);
+            s.ent[e] = r;
             s.tsize[e] = pos_table_size(a.n_cmp[g], a.pos_cap);
-            s.bnd[e] = !(bb[0] > a.geo.gb && bb[1] < a.geo.M - a.geo.gb && bb[2] > a.geo.gb &&
-                         bb[3] < a.geo.M - a.geo.gb && bb[4] > a.geo.gb && bb[5] < a.geo.M - a.geo.gb);
-            s.bbox[6 * e + 0] = INT_MAX; s.bbox[6 * e + 1] = INT_MIN;
-            s.bbox[6 * e + 2] = INT_MAX; s.bbox[6 * e + 3] = INT_MIN;
-            s.bbox[6 * e + 4] = INT_MAX; s.bbox[6 * e + 5] = INT_MIN;
+            s.pmask[e][0] = s.pmask[e][1] = 0u;
+            s.ucol[e] = 0xFF;
         }
         if (threadIdx.x < 8) s.umask[threadIdx.x] = 0u;
+        if (threadIdx.x == 8) s.nu[0] = 0;
         __syncthreads();
         // values of every covering box over the tile (-inf outside the box), copied with
         // cp.async so that no thread waits on one load before issuing the next
-        {
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-            for (int e = warp; e < m; e += nw) {
-                const Box B = load_box(s.box + 6 * e);
-                const T* src = a.in.data + s.off[e];
-#pragma unroll
-                for (int vv = 0; vv < kTV; vv += 32) {
-                    const int v = vv + lane;
-                    const int x = X0 + v % kTX, y = Y0 + (v / kTX) % kTY, z = Z0 + v / (kTX * kTY);
-                    if (x >= B.x0 && x < B.x1 && y >= B.y0 && y < B.y1 && z >= B.z0 && z < B.z1)
-                        cp_async_elem(s.val + e * kVS + v, src + B.at(y, x, z));
-                    else
-                        s.val[e * kVS + v] = NEG;
+        for (int e = warp; e < m; e += kThreads / 32) {
+            const Entry& r = s.ent[e];
+            const T* src = a.in.data + r.in + (dy * r.nx + dx);
+            T* dst = s.val + e * kVS + lane;
+            if ((r.cover[0] >> lane) & 1u) cp_async_elem(dst, src);
+            else dst[0] = NEG;
+            if ((r.cover[1] >> lane) & 1u) cp_async_elem(dst + 32, src + r.nxy);
+            else dst[32] = NEG;
+        }
+        // the boundary distance of this voxel (box.cpp:997-1088): a voxel at least gb from
+        // every face of the boundary grain's zone gets an all-negative distance <= -gb,
+        // which changes nothing
+        if (threadIdx.x < kTV) {
+            const int v = threadIdx.x, x = X0 + v % kTX, y = Y0 + (v / kTX) % kTY, z = Z0 + v / (kTX * kTY);
+            const int lo_in = 2 * a.geo.gb - 1, hi_in = a.geo.M - 1 - 2 * a.geo.gb;
+            T thr = NEG, set = T(0);
+            bool unk = false;
+            if (!(x >= lo_in && x <= hi_in && y >= lo_in && y <= hi_in && z >= lo_in && z <= hi_in)) {
+                double d = 0.0;
+                unk = !bc_assign(y, x, z, a.geo.M, a.geo.gb, d);
+                if (!unk && d > -a.geo.gb) {
+                    thr = not_below<T>(d * a.geo.h);
+                    set = (T)(d * a.geo.h);
                 }
             }
+            s.bthr[v] = thr;
+            s.bset[v] = set;
+            s.bunk[v] = unk;
         }
         cp_async_wait_all();
         __syncthreads();
         // per voxel: the kTop largest values > -1.  The kParts lanes of a voxel are
         // neighbours in one warp; each keeps the top of every kParts-th box, then two
-        // shuffle rounds merge their lists (a bitonic merge of two sorted lists of kTop).
+        // shuffle rounds merge their lists into the first lane's.
         {
-            const int lane = threadIdx.x & 31;
-            const int part = lane & (kParts - 1), v = (threadIdx.x >> 5) * (32 / kParts) + (lane / kParts);
+            const int part = lane & (kParts - 1), v = warp * (32 / kParts) + (lane / kParts);
             T tv[kTop];
             int ti[kTop];
 #pragma unroll
-            for (int k = 0; k < kTop; k++) { tv[k] = NEG; ti[k] = 0xFF; }
-            int nc = 0;
-            for (int e = part; e < m; e += kParts) {
-                const T w = s.val[e * kVS + v];
-                if (!(w > T(-1))) continue;
-                nc++;
-                top_insert(tv, ti, w, e);
-            }
+            for (int k = 0; k < kTop; k++) { tv[k] = T(-1); ti[k] = 0xFF; }
+            for (int e = part; e < m; e += kParts) top_insert(tv, ti, s.val[e * kVS + v], e);
 #pragma unroll
             for (int o = 1; o < kParts; o <<= 1) {
                 T pv[kTop];
                 int pi[kTop];
 #pragma unroll
                 for (int k = 0; k < kTop; k++) {
-                    pv[k] = __shfl_xor_sync(0xffffffffu, tv[k], o);
-                    pi[k] = __shfl_xor_sync(0xffffffffu, ti[k], o);
+                    pv[k] = __shfl_down_sync(0xffffffffu, tv[k], o);
+                    pi[k] = __shfl_down_sync(0xffffffffu, ti[k], o);
                 }
-                nc += __shfl_xor_sync(0xffffffffu, nc, o);
-                // both lanes merge (lower part's list, higher part's list) alike
-                const bool low = (lane & o) == 0;
-                T av[kTop], bv[kTop];
-                int ai[kTop], bi[kTop];
 #pragma unroll
-                for (int k = 0; k < kTop; k++) {
-                    av[k] = low ? tv[k] : pv[k];
-                    ai[k] = low ? ti[k] : pi[k];
-                    bv[k] = low ? pv[k] : tv[k];
-                    bi[k] = low ? pi[k] : ti[k];
-                }
-                // the kTop largest of both: max(a[k], b[kTop-1-k]), a bitonic sequence
-#pragma unroll
-                for (int k = 0; k < kTop; k++) {
-                    const bool ta = !(bv[kTop - 1 - k] > av[k]);
-                    tv[k] = ta ? av[k] : bv[kTop - 1 - k];
-                    ti[k] = ta ? ai[k] : bi[kTop - 1 - k];
-                }
-                // sorted descending by a bitonic half-cleaner cascade
-#pragma unroll
-                for (int j = kTop / 2; j > 0; j >>= 1)
-#pragma unroll
-                    for (int k = 0; k < kTop; k++)
-                        if ((k & j) == 0 && tv[k + j] > tv[k]) {
-                            const T t = tv[k]; tv[k] = tv[k + j]; tv[k + j] = t;
-                            const int u = ti[k]; ti[k] = ti[k + j]; ti[k + j] = u;
-                        }
+                for (int k = 0; k < kTop; k++) top_insert(tv, ti, pv[k], pi[k]);
             }
             if (part == 0) {
 #pragma unroll
                 for (int k = 0; k < kTop; k++) {
-                    s.topv[k * kTV + v] = tv[k];
+                    s.topv[k * kTV + v] = ti[k] != 0xFF ? tv[k] : NEG;
                     s.topi[k * kTV + v] = (unsigned char)ti[k];
-                    if (ti[k] != 0xFF) atomicOr(s.umask + (ti[k] >> 5), 1u << (ti[k] & 31));
                 }
-                s.ncand[v] = nc;
-                // A voxel at least gb from every face of the boundary grain's zone gets an
-                // all-negative distance <= -gb from bc_assign, which changes nothing.
-                const int x = X0 + v % kTX, y = Y0 + (v / kTX) % kTY, z = Z0 + v / (kTX * kTY);
-                const int lo_in = 2 * a.geo.gb - 1, hi_in = a.geo.M - 1 - 2 * a.geo.gb;
-                s.deep[v] = x >= lo_in && x <= hi_in && y >= lo_in && y <= hi_in && z >= lo_in && z <= hi_in;
+                // a column of pos for every entry among some voxel's two largest
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    if (ti[k] != 0xFF && !((s.umask[ti[k] >> 5] >> (ti[k] & 31)) & 1u)) {
+                        const unsigned bit = 1u << (ti[k] & 31);
+                        if (!(atomicOr(s.umask + (ti[k] >> 5), bit) & bit)) {
+                            const int col = atomicAdd(s.nu, 1);
+                            if (col < kUCap) {
+                                s.ulist[col] = (unsigned char)ti[k];
+                                s.ucol[ti[k]] = (unsigned char)col;
+                            }
+                        }
+                    }
             }
         }
         __syncthreads();
-        // the columns of pos the pair loop reads: every entry that is among some voxel's
-        // kTop candidates.  pos[a][b] = position of b in a's list, from a's position
-        // table; kBatch lookups advance together, each round issuing all their next probes
-        if (threadIdx.x < 32) {
-            int nu = 0;
-            for (int b0 = 0; b0 < m; b0 += 32) {
-                const int b = b0 + threadIdx.x;
-                const bool in_u = b < m && ((s.umask[b >> 5] >> (b & 31)) & 1u);
-                const unsigned bal = __ballot_sync(0xffffffffu, in_u);
-                const int r = nu + __popc(bal & ((1u << threadIdx.x) - 1));
-                if (in_u) s.ulist[r] = (unsigned char)b;
-                if (b < m) s.ucol[b] = (in_u && r < kUCap) ? (unsigned char)r : (unsigned char)0xFF;
-                nu += __popc(bal);
-            }
-            if (threadIdx.x == 0) s.nu[0] = nu;
-        }
-        __syncthreads();
+        // pos[a][column of b] = position of b in a's list, from a's position table; kBatch
+        // lookups advance together, each round issuing all their next probes.  Columns beyond
+        // kUCap are looked up when needed.
         {
-            constexpr int kBatch = 4;
-            const int nu = min(s.nu[0], kUCap);  // columns beyond kUCap are looked up when needed
+            constexpr int kBatch = 2;
+            const int nu = min(s.nu[0], kUCap);
             const int mm = m * nu;
             for (int q0 = 0; q0 < mm; q0 += kBatch * kThreads) {
                 unsigned long long e[kBatch];
@@ -475,9 +554,9 @@ __global__ void __launch_bounds__(kThreads, 4) compare_kernel(CompareArgs<T> a) 
                     h[u] = mask[u] = id[u] = 0;
                     e[u] = 0;
                     if (live[u]) {
-                        tab[u] = a.pos_table + (long long)s.id[ea] * a.pos_cap;
+                        tab[u] = a.pos_table + (long long)s.ent[ea].id * a.pos_cap;
                         mask[u] = (unsigned)s.tsize[ea] - 1;
-                        id[u] = s.id[eb];
+                        id[u] = s.ent[eb].id;
                         h[u] = pos_home(id[u], s.tsize[ea]);
                         e[u] = __ldg(tab[u] + h[u]);
                     }
@@ -504,106 +583,72 @@ __global__ void __launch_bounds__(kThreads, 4) compare_kernel(CompareArgs<T> a) 
             }
         }
         __syncthreads();
-        // every (grain, voxel) pair of the tile
-        const double lim = 0.7 * a.geo.delta;
-        for (int q = threadIdx.x; q < m * kTV; q += blockDim.x) {
-            const int ea = q / kTV, v = q % kTV;
-            const T in = s.val[ea * kVS + v];
-            const int x = X0 + v % kTX, y = Y0 + (v / kTX) % kTY, z = Z0 + v / (kTX * kTY);
-            bool positive = false;
-            // else the voxel is outside this grain's box, or (recalculateIDLocal) the grain
-            // does not exist and executeComparison leaves it alone
-            if (in != NEG && (a.set_comparison || a.exists[s.id[ea]])) {
-            // the first listed neighbour among the largest values, ties to the earliest position
-            int best = -1;
-            unsigned short bpos = kNotListed;
-            T level = NEG;
-            bool decided = false;
-            int k = 0;
-            for (; k < kTop; k++) {
-                const int eb = s.topi[k * kTV + v];
-                if (eb == 0xFF) break;
-                const T w = s.topv[k * kTV + v];
-                if (best >= 0 && !(w == level)) { decided = true; break; }
-                if (eb == ea) continue;
-                const int col = s.ucol[eb];
-                const unsigned short p = col != 0xFF ? s.pos[ea * kUCap + col]
-                                                     : list_position(a, s.id[ea], s.tsize[ea], s.id[eb]);
-                if (p == kNotListed) continue;
-                if (best < 0 || p < bpos) { best = eb; bpos = p; level = w; }
-            }
-            // decided anyway when every covering candidate was among those examined
-            if (!decided && s.ncand[v] <= k) decided = true;
-            if (!decided) {  // full scan of the tile's boxes at this voxel
-                best = -1;
-                bpos = kNotListed;
-                level = NEG;
-                for (int eb = 0; eb < m; eb++) {
-                    if (eb == ea) continue;
-                    const T w = s.val[eb * kVS + v];
-                    if (!(w > T(-1))) continue;
-                    if (best >= 0 && w < level) continue;
-                    const int col = s.ucol[eb];
-                    const unsigned short p = col != 0xFF ? s.pos[ea * kUCap + col]
-                                                         : list_position(a, s.id[ea], s.tsize[ea], s.id[eb]);
-                    if (p == kNotListed) continue;
-                    if (best < 0 || w > level || (w == level && p < bpos)) { best = eb; bpos = p; level = w; }
-                }
-            }
-            const uint32_t ga = s.id[ea];
-            const Box A = load_box(s.box + 6 * ea);
-            const long long f = A.at(y, x, z);
-            T cmpv;
-            uint32_t idv;
-            if (best >= 0) {
-                cmpv = s.val[best * kVS + v];
-                idv = s.id[best];
-            } else {  // no listed neighbour covers the voxel: value -1, IDLocal kept
-                cmpv = T(-1);
-                const Box Bold = load_box(a.idbox_old + 6 * ga);
-                idv = f < Bold.count() ? a.id_old[a.idoff_old[ga] + f] : 0u;
-            }
-            if (s.bnd[ea] && !s.deep[v]) {  // the boundary condition near the zone's faces
-                const double d = bc_dist(A, y, x, z, a.geo.M, a.geo.gb);
-                if (d > -a.geo.gb)
-                    if (d * a.geo.h > (double)cmpv) {
-                        cmpv = (T)(d * a.geo.h);
-                        idv = 0;
+        // every (grain, voxel) pair of the tile: a thread keeps its voxel, a warp shares the
+        // entry (kTV and kThreads are multiples of 64)
+        {
+            const int v = threadIdx.x % kTV, dz = v / 32;
+            const T w0 = s.topv[v], w1 = s.topv[kTV + v], w2 = s.topv[2 * kTV + v];
+            const int i0 = s.topi[v], i1 = s.topi[kTV + v];
+            const int c0 = i0 != 0xFF ? s.ucol[i0] : 0xFF, c1 = i1 != 0xFF ? s.ucol[i1] : 0xFF;
+            const uint32_t g0 = i0 != 0xFF ? s.ent[i0].id : 0u, g1 = i1 != 0xFF ? s.ent[i1].id : 0u;
+            const T bthr = s.bthr[v], bset = s.bset[v];
+            const bool bunk = s.bunk[v];
+            for (int ea = threadIdx.x / kTV; ea < m; ea += kThreads / kTV) {
+                const Entry& r = s.ent[ea];
+                const unsigned flags = r.flags;
+                bool positive = false;
+                // else the voxel is outside this grain's box, or (recalculateIDLocal) the
+                // grain does not exist and executeComparison leaves it alone
+                if (((r.cover[dz] >> lane) & 1u) && (flags & kActive)) {
+                    const T in = s.val[ea * kVS + v];
+                    const int f = dz * r.nxy + dy * r.nx + dx;
+                    // the largest other value, decided when it is listed and the next differs
+                    const bool self = i0 == ea;
+                    const int col = self ? c1 : c0;
+                    T cmpv = self ? w1 : w0;
+                    uint32_t idv = self ? g1 : g0;
+                    const T next = self ? w2 : w1;
+                    if (col == 0xFF || next == cmpv || s.pos[ea * kUCap + col] == kNotListed) {
+                        const Neighbour<T> n = slow_pair(smem_raw, a, ea, v, m, Y0 + dy, X0 + dx, Z0 + dz);
+                        cmpv = n.value;
+                        idv = n.id;
                     }
-            }
-            T res;
-            if (!a.set_comparison) res = cmpv;
-            else if (in_band(in, lim)) res = T(0.5) * (in - cmpv);
-            else res = in;
-            a.out.data[s.outoff[ea] + f] = res;
-            a.id_new[s.idoff[ea] + f] = idv;
-            positive = a.set_comparison && res >= 0;
-            }
-            // new bounding box (executeSetComparison, box.cpp:858-877), reduced over the warp
-            // first: its 32 lanes hold the same entry (kTV and blockDim are multiples of 64)
-            if (__ballot_sync(0xffffffffu, positive)) {
-                const int x0 = __reduce_min_sync(0xffffffffu, positive ? x : INT_MAX);
-                const int x1 = __reduce_max_sync(0xffffffffu, positive ? x : INT_MIN);
-                const int y0 = __reduce_min_sync(0xffffffffu, positive ? y : INT_MAX);
-                const int y1 = __reduce_max_sync(0xffffffffu, positive ? y : INT_MIN);
-                const int z0 = __reduce_min_sync(0xffffffffu, positive ? z : INT_MAX);
-                const int z1 = __reduce_max_sync(0xffffffffu, positive ? z : INT_MIN);
-                if ((threadIdx.x & 31) == 0) {
-                    int* bb = s.bbox + 6 * ea;
-                    atomicMin(bb + 0, x0); atomicMax(bb + 1, x1);
-                    atomicMin(bb + 2, y0); atomicMax(bb + 3, y1);
-                    atomicMin(bb + 4, z0); atomicMax(bb + 5, z1);
+                    if (flags & kBoundary) {  // the boundary condition near the zone's faces
+                        if (bunk) {  // the value of an earlier voxel of this box's loop
+                            const double d = carried_dist(a, r.id, Y0 + dy, X0 + dx, Z0 + dz);
+                            if (d > -a.geo.gb)
+                                if (d * a.geo.h > (double)cmpv) {
+                                    cmpv = (T)(d * a.geo.h);
+                                    idv = 0;
+                                }
+                        } else if (cmpv < bthr) {
+                            cmpv = bset;
+                            idv = 0;
+                        }
+                    }
+                    T res;
+                    if (!a.set_comparison) res = cmpv;
+                    else if (fabs(in) < lim) res = T(0.5) * (in - cmpv);
+                    else res = in;
+                    a.out.data[r.out + f] = res;
+                    a.id_new[r.idn + f] = idv;
+                    positive = a.set_comparison && res >= 0;
                 }
+                // the voxels of the new bounding box (executeSetComparison, box.cpp:858-877)
+                const unsigned bal = __ballot_sync(0xffffffffu, positive);
+                if (bal && lane == 0) s.pmask[ea][dz] = bal;
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < m; e += blockDim.x) {
-            const int* bb = s.bbox + 6 * e;
-            if (bb[0] == INT_MAX) continue;
-            int* nb = a.newbox + 6 * s.id[e];
-            atomicMin(nb + 0, bb[0]); atomicMax(nb + 1, bb[1]);
-            atomicMin(nb + 2, bb[2]); atomicMax(nb + 3, bb[3]);
-            atomicMin(nb + 4, bb[4]); atomicMax(nb + 5, bb[5]);
+        for (int e = threadIdx.x; e < m; e += kThreads) {
+            const unsigned p0 = s.pmask[e][0], p1 = s.pmask[e][1], p = p0 | p1;
+            if (!p) continue;
+            unsigned row = p | (p >> 16);
+            row = (row | (row >> 8)) & 0xFFu;  // the x of any row; a byte per y
+            int* nb = a.newbox + 6 * s.ent[e].id;
+            atomicMin(nb + 0, X0 + __ffs(row) - 1); atomicMax(nb + 1, X0 + 31 - __clz(row));
+            atomicMin(nb + 2, Y0 + ((__ffs(p) - 1) >> 3)); atomicMax(nb + 3, Y0 + ((31 - __clz(p)) >> 3));
+            atomicMin(nb + 4, Z0 + (p0 ? 0 : 1)); atomicMax(nb + 5, Z0 + (p1 ? 1 : 0));
         }
         __syncthreads();
     }
@@ -622,10 +667,7 @@ __global__ void newbox_init_kernel(int G, const int* present, const int* exists,
 }  // namespace
 
 size_t compare_smem_bytes(int mcap, bool fp64) {
-    const size_t e = fp64 ? 8 : 4;
-    return 24 * (size_t)mcap + e * (size_t)mcap * kVS + e * kTV * kTop + 4 * (size_t)mcap +
-           48 * (size_t)mcap + 4 * (size_t)mcap + 4 * kTV + 48 + 2 * (size_t)mcap * kUCap + 512 +
-           kTV * kTop + kTV + (size_t)mcap + 64;
+    return fp64 ? tile_smem_bytes<double>(mcap) : tile_smem_bytes<float>(mcap);
 }
 
 long long bin_capacity(int G, int side) {

@@ -184,6 +184,47 @@ def test_loop_fp64_bitexact(gpu, oracle, name, steps):
             assert ob == gb_ and np.array_equal(osdf, gsdf), f"final SDF grain {g}"
 
 
+@pytest.mark.parametrize("border", [4, 7])
+@pytest.mark.parametrize("lists", ["reversed", "thinned"])
+def test_comparison_of_ties_and_unlisted_neighbours_bitexact(gpu, oracle, border, lists):
+    """A lattice of equal cubes, whose fields tie along every symmetry plane (the earliest
+    list position decides), with lists in descending order, or with 40% of their members
+    left out and some lists empty (unlisted candidates and voxels no listed neighbour
+    covers keep their IDLocal): the fields and IDs equal the oracle's bit for bit."""
+    n, c = 4, 6
+    N, G = n * c, n ** 3
+    ax = np.arange(N) // c
+    lab = (1 + ax[None, None, :] + n * ax[None, :, None] + n * n * ax[:, None, None]).astype(np.uint32)
+    cube = np.array([[x * c, x * c + c - 1, y * c, y * c + c - 1, z * c, z * c + c - 1]
+                     for z in range(n) for y in range(n) for x in range(n)], np.int32)
+    counts = np.full(G, c ** 3, np.int64)
+    gh = gpu.GrainHandler(N, border, 0.2, G, precision=0)
+    gh.load(lab, cube, counts)
+    gh.default_lists()
+    rng = np.random.default_rng(5)
+    rows = []
+    for g in range(1, G + 1):
+        r = gh.comparison_list(g)
+        rows.append(r[::-1] if lists == "reversed" else (r[rng.random(r.size) < 0.6] if g % 9 else r[:0]))
+    off = np.concatenate([[0, 0], np.cumsum([r.size for r in rows])]).astype(np.int64)
+    ids = np.concatenate(rows).astype(np.uint32)
+    gh.set_lists(off, ids)
+    osim = oracle.OracleSim(N, border, 0.2, lab, cube, counts, lists=(off, ids))
+    for s in range(3):
+        assert gh.step()["grain_count"] == osim.step(), f"step {s}"
+        st = gh.stats()
+        for g in range(1, G + 1):
+            inf = osim.info(g)
+            assert bool(st.exists[g]) == inf["exists"], f"step {s} grain {g}"
+            assert np.array_equal(gh.comparison_list(g), osim.comparison_list(g)), f"step {s} grain {g}: list"
+            if inf["exists"]:
+                assert tuple(st.boxes[g]) == inf["box"] and st.volume[g] == inf["volume"], f"step {s} grain {g}"
+                ob, oid = osim.idlocal(g)
+                gb, gid = gh.idlocal(g)
+                assert ob == gb and np.array_equal(oid, gid), f"step {s} grain {g}: IDLocal"
+                assert np.array_equal(osim.sdf(g)[1], gh.sdf(g)[1]), f"step {s} grain {g}: field"
+
+
 def test_loop_mixed_volume_tolerance(gpu, oracle):
     c, gh, osim = _pair(gpu, oracle, "border10", precision=1)
     worst = 0.0
