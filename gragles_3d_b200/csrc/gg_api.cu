@@ -407,7 +407,8 @@ int correct_convolution(gg_ctx* ctx) {
     c.el = ctx->el;
     c.ph = physics(ctx);
     c.err = ctx->d_err;
-    launch_work_order(ctx->work, ctx->G, ctx->d_toff_one, ctx->d_box[p], correction_item_voxels(), ctx->stream);
+    c.item_vox = correction_item_voxels(*ctx->h_total_vox, ctx->num_sms);  // the last step's voxels
+    launch_work_order(ctx->work, ctx->G, ctx->d_toff_one, ctx->d_box[p], c.item_vox, ctx->stream);
     c.order = ctx->work.order;
     c.item_off = ctx->work.item_off;
     c.queue = ctx->work.queue;

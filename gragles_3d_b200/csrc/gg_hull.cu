@@ -15,10 +15,10 @@
 //     as the reference does (including its ID-list quirks), and writes the elements in
 //     search order with their barycenter segments, bounding boxes and an ID -> elements
 //     index.
-//   correction_kernel: a CTA per grain, with the grain's element index, element boxes
-//     and FP32 barycenters staged in shared memory; pass by pass over runs of the box's
-//     voxels, those with |input| < delta are grouped by IDLocal neighbour, and a warp
-//     takes 32 voxels of one neighbour at a time.  The winner of the reference's search is the least (distance, element
+//   correction_kernel: a CTA per run of a grain's box voxels, with the grain's element index,
+//     element boxes and FP32 barycenters staged in shared memory; pass by pass, the voxels
+//     with |input| < delta are grouped by IDLocal neighbour, and a warp takes 64 voxels of
+//     one neighbour at a time.  The winner of the reference's search is the least (distance, element
 //     index) over the barycenters of the elements holding that neighbour.  The warp
 //     finds it with an FP32 filter -- per barycenter p, q = |p'|^2 - 2 v'.p' (three FMAs
 //     on coordinates relative to an integer origin), minimised per element -- that
@@ -980,7 +980,7 @@ __global__ void __launch_bounds__(32) elements_kernel(ElementArgs a) {
             // every barycenter to its element's run: lane-parallel over the grouped array,
             // barycenter i of list k (the last list whose first barycenter is <= i) going to
             // lflat[k] + (i - off[k])
-            float* pf = reinterpret_cast<float*>(a.el.ebf + (long long)g * a.el.flat_cap);
+            float4* pf = a.el.ebf + (long long)g * a.el.flat_cap;
             int* pidx = a.el.eidx + (long long)g * a.el.flat_cap;
             float r2 = 0.f;
             // the barycenter of the lane's next index is loaded while this one is placed
@@ -1004,11 +1004,7 @@ __global__ void __launch_bounds__(32) elements_kernel(ElementArgs a) {
                 if (dst < 0 || dst >= nflat) continue;  // a list no element holds
                 const double dx = b0 - org[0], dy = b1 - org[1], dz = b2 - org[2];
                 const double w = dx * dx + dy * dy + dz * dz;
-                float* pp = pf + 8 * (dst >> 1) + (dst & 1);  // pair layout: x0 x1 y0 y1 z0 z1 w0 w1
-                pp[0] = (float)dx;
-                pp[2] = (float)dy;
-                pp[4] = (float)dz;
-                pp[6] = (float)w;
+                pf[dst] = make_float4((float)dx, (float)dy, (float)dz, (float)w);
                 pidx[dst] = i;
                 r2 = fmaxf(r2, (float)w);
                 const int e = S.fill[lo];  // the element list lo went to (emit)
@@ -1039,11 +1035,7 @@ __global__ void __launch_bounds__(32) elements_kernel(ElementArgs a) {
                 for (int e = lane; e < S.ne; e += 32) {
                     const int n = E[e].pcount, dst = E[e].pbase + n;
                     if ((n & 1) && dst >= 0 && dst < nflat) {
-                        float* pp = pf + 8 * (dst >> 1) + (dst & 1);
-                        pp[0] = 0.f;
-                        pp[2] = 0.f;
-                        pp[4] = 0.f;
-                        pp[6] = kPadQ;
+                        pf[dst] = make_float4(0.f, 0.f, 0.f, kPadQ);
                         pidx[dst] = -1;
                     }
                 }
@@ -1079,12 +1071,26 @@ constexpr float kInf = 3.0e38f;
 constexpr int kSPts = 2304;           // barycenters staged in shared memory (more: read from HBM)
 constexpr int kSElem = kLMax;         // elements per grain: one per distinct list at most
 constexpr int kSPairs = kPairMax;     // the index's (element, ID) pairs per grain
+constexpr int kCPackets = kCVox / kPacket + kIdxMax;  // packets of a pass: full ones, and one part-full a neighbour
+constexpr int kSurv = 56;             // barycenters a warp buffers
 static_assert(kSElem <= 0xFFFF && kSPairs <= 0xFFFF, "16-bit element and pair indices");
 static_assert(kSPairs % 8 == 0, "pair lists are copied 16 bytes at a time");
 
-// One grain's search data, staged once per grain, and the slice pass's voxel groups.
+// One warp's buffer of the barycenters a packet still has to look at, grouped by the element
+// they belong to; an odd group is padded by one entry (w = kPadQ).
+struct alignas(16) Survivors {
+    float f[4 * kSurv];                // in pairs: x0 x1 y0 y1 | z0 z1 w0 w1
+    unsigned short cand[kSurv / 2];    // group: candidate (position in the neighbour's element list)
+    unsigned short end[kSurv / 2];     // group: end of its entries
+};
+
+// One grain's search data, staged once per work item, and the pass's voxel groups.
 struct CorrSmem {
-    float4 pts[kSPts];            // FP32 barycenters, element by element, in pairs (ebf)
+    float4 pts[kSPts];            // FP32 barycenters, element by element (ebf)
+    union {
+        unsigned short vd[kCVox];  // dense neighbour index of the pass's voxels, kNoD: no search; once
+        Survivors surv[kCThreads / 32];  // they are grouped, the warps' buffers
+    };
     float box[kSElem][6];         // element boxes relative to the origin, rounded outward
     int2 erun[kSElem];            // element e's run in ebf: (first, count), both even
     alignas(16) unsigned short pairs[kSPairs];  // the index's element lists (search order per ID)
@@ -1092,7 +1098,7 @@ struct CorrSmem {
     unsigned short hden[kCHash];
     int2 drng[kIdxMax];           // dense index d -> its elements in pairs
     int dcnt[kIdxMax], doff[kIdxMax], dcur[kIdxMax], dpk[kIdxMax + 1];
-    unsigned short vd[kCVox];     // dense neighbour index of the pass's voxels, kNoD: no search
+    unsigned short pkd[kCPackets];  // packet -> dense index
     unsigned short vlist[kCVox];  // pass voxels grouped by neighbour
     int next;                     // the work item this CTA fetched
     int pk_next;                  // the pass's next unclaimed packet
@@ -1102,12 +1108,6 @@ struct CorrSmem {
 // |p'|^2 - 2 v'.p' = |v' - p'|^2 - |v'|^2.
 __device__ __forceinline__ float qval(const float4 p, float ax, float ay, float az) {
     return fmaf(az, p.z, fmaf(ay, p.y, fmaf(ax, p.x, p.w)));
-}
-
-// Barycenter i of the pair layout (x0 x1 y0 y1 | z0 z1 w0 w1 per pair) as (x, y, z, w).
-__device__ __forceinline__ float4 pt_at(const float4* pts, int i) {
-    const float* f = reinterpret_cast<const float*>(pts + 2 * (i >> 1)) + (i & 1);
-    return make_float4(f[0], f[2], f[4], f[6]);
 }
 
 // Two FP32 lanes packed in 64 bits: the operands of the packed FMA.
@@ -1133,25 +1133,6 @@ __device__ __forceinline__ float min_of(float m, unsigned long long r) {
     return d;
 }
 
-// The least q, for each of a lane's V voxels, over the n (even) barycenters of a run
-// starting at pair boundary `first`: two barycenters per packed FMA chain, the same
-// three roundings per barycenter as qval.  Each loaded pair serves all V voxels.
-template <int V>
-__device__ __forceinline__ void run_min(const float4* pts, int first, int n, const unsigned long long (&A2)[V],
-                                        const unsigned long long (&B2)[V], const unsigned long long (&C2)[V],
-                                        float (&m)[V]) {
-    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(pts + first);  // 2 per pair
-    const int np = n >> 1;
-#pragma unroll
-    for (int u = 0; u < V; u++) m[u] = kInf;
-#pragma unroll 2
-    for (int i = 0; i < np; i++) {
-        const ulonglong2 xy = p[2 * i], zw = p[2 * i + 1];
-#pragma unroll
-        for (int u = 0; u < V; u++) m[u] = min_of(m[u], fma2(C2[u], zw.x, fma2(B2[u], xy.y, fma2(A2[u], xy.x, zw.y))));
-    }
-}
-
 // The near-tie case: the barycenters whose q is within the band, measured with the
 // reference's FP64 distance (Vector3d::squaredNorm, c0 + (c1 + c2)) and kept only when
 // strictly nearer, visiting elements in search order and each element's barycenters in
@@ -1161,7 +1142,7 @@ __device__ __forceinline__ void run_min(const float4* pts, int first, int n, con
 // `band` marks (bit c, when count <= 32) the candidates whose least q came within the band
 // of the best so far when they were scanned: a superset of those within the final band,
 // the only ones that can hold such a barycenter; the rest are not visited.
-__device__ int exact_winner(const CorrSmem& S, const float4* pts, int first, int count, int ne,
+__device__ __noinline__ int exact_winner(const CorrSmem& S, const float4* pts, int first, int count, int ne,
                             const int* __restrict__ eidx, const double* __restrict__ eb, double x, double y, double z,
                             float ax, float ay, float az, float limit, unsigned band) {
     double bd = 10000000.0;
@@ -1172,7 +1153,7 @@ __device__ int exact_winner(const CorrSmem& S, const float4* pts, int first, int
         if (e >= ne) continue;
         const int2 r = S.erun[e];  // the element's barycenters in order (a padding entry: q = kInf)
         for (int i = r.x; i < r.x + r.y; i++) {
-            if (qval(pt_at(pts, i), ax, ay, az) > limit) continue;
+            if (qval(pts[i], ax, ay, az) > limit) continue;
             const int src = eidx[i];
             if (src < 0) continue;
             const double d = sqdist3(x, y, z, eb + 3 * (long long)src);
@@ -1189,7 +1170,7 @@ __device__ int exact_winner(const CorrSmem& S, const float4* pts, int first, int
 // of each element the band holds, keeping the least FP64 distance and, among equal
 // ones, the first in its own order; the warp then reduces on (distance, element position
 // c, barycenter) -- the first in search order among the least, as the sequential walk.
-__device__ int exact_winner_warp(const CorrSmem& S, const float4* pts, int first, int count, int ne,
+__device__ __noinline__ int exact_winner_warp(const CorrSmem& S, const float4* pts, int first, int count, int ne,
                                  const int* __restrict__ eidx, const double* __restrict__ eb, int i, int j, int k,
                                  float4 org, float limit, unsigned band) {
     const int lane = threadIdx.x & 31;
@@ -1203,7 +1184,7 @@ __device__ int exact_winner_warp(const CorrSmem& S, const float4* pts, int first
         if (e >= ne) continue;
         const int2 r = S.erun[e];
         for (int t = lane; t < r.y; t += 32) {
-            if (qval(pt_at(pts, r.x + t), ax, ay, az) > limit) continue;
+            if (qval(pts[r.x + t], ax, ay, az) > limit) continue;
             const int src = eidx[r.x + t];
             if (src < 0) continue;
             const double d = sqdist3(x, y, z, eb + 3 * (long long)src);
@@ -1225,82 +1206,180 @@ __device__ int exact_winner_warp(const CorrSmem& S, const float4* pts, int first
     return bkey == 0x7FFFFFFF ? -1 : S.pairs[first + (bkey >> 20)];
 }
 
-// Lower bound of q over a box [lo, hi] (relative, rounded outward) for the voxel v':
-// |v' - box|^2 in FP32, scaled down past its rounding, - |v'|^2 - eps.
-__device__ __forceinline__ float box_bound(float vx, float vy, float vz, float vv, float lx, float ly, float lz,
-                                           float hx, float hy, float hz, float eps) {
-    const float dx = vx < lx ? lx - vx : (vx > hx ? vx - hx : 0.f);
-    const float dy = vy < ly ? ly - vy : (vy > hy ? vy - hy : 0.f);
-    const float dz = vz < lz ? lz - vz : (vz > hz ? vz - hz : 0.f);
-    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    return d2 * (1.f - 1.0f / 1048576.f) - vv - eps;
-}
-
 // The elements whose (energy, mobility) a lane's V voxels (i, j, k) take: the
 // reference's winner among the elements S.pairs[first, first + count) (-1: none,
 // weight (1, 1)).  All lanes of the warp call it with the same elements (a packet of one
-// neighbour).  Per voxel, each element's least q is compared with the best and
-// second-best so far; when the best element beats every other by more than eps2 (twice
-// the filter's error bound) it is the reference's winner, else the near tie is settled
-// in FP64 (exact_winner).  Elements are taken in reverse search order, so the grain
-// boundary (last in search order, and the usual winner) sets a tight best first, and an
-// element is skipped when no voxel of the warp can come within the band of its best
-// through the element's box.
+// neighbour).  Per voxel, the least q and the least q of the other elements are kept; when
+// the best element beats every other by more than eps2 (twice the filter's error bound) it
+// is the reference's winner, else the near tie is settled in FP64 (exact_winner).
+//
+// Most barycenters cannot win for any voxel of the packet, and the warp finds those that can
+// with its lanes over the barycenters instead of the voxels.  With c the centre of the
+// packet's voxels, D their half extents and p0 any barycenter,
+//   q_v(p) - q_v(p0) = q_c(p) - q_c(p0) - 2 (v - c).(p - p0) >= q_c(p) - q_c(p0) - 2 D.|p - p0|,
+// so a p whose right-hand side is positive by more than `margin` is behind p0 by more than
+// eps2 for all of them, as q is computed: 2 eps2 for the errors of q_v(p) and q_v(p0) and the
+// band itself, eps2 for those of q_c, and 3 eps2 for the rounding of the bound (each below
+// 28 R^2 2^-24 < eps2).  The same test on an element's box drops it whole; p0 is the nearest to
+// c of the last element in search order, the grain boundary, usually the winner's.  The
+// projection point lies far from the hull (a median of 53 voxels), where a packet spans a
+// small angle: of 146 candidate barycenters a packet keeps 23 (256^3 / 20,000 grains).  Every
+// voxel against every candidate, two at a time with packed FMAs, the kernel took 17.4 ms there
+// (issue-bound) and 15 ms for 30 grains of 90^3 voxels (5,500 candidates a packet, 750 kept);
+// now 14.1 and 5.5 ms.
 template <int V>
-__device__ __forceinline__ void search_packet(const CorrSmem& S, const float4* pts, int first, int count,
+__device__ __forceinline__ void search_packet(const CorrSmem& S, Survivors& W, const float4* pts, int first, int count,
                                               const bool (&active)[V], const int (&ii)[V], const int (&jj)[V],
                                               const int (&kk)[V], float4 org, float eps2, int ne,
                                               const int* __restrict__ eidx, const double* __restrict__ eb, int* err,
                                               int (&win)[V]) {
-    float vx[V], vy[V], vz[V], vv[V], best[V], second[V];
-    unsigned long long A2[V], B2[V], C2[V];
-    int beste[V];
+    const int lane = threadIdx.x & 31;
+    unsigned long long ax[V], ay[V], az[V];  // -2 v', in both halves
+    float best[V], second[V];
+    int bestc[V];
     unsigned band[V];  // candidates within the band of the best when scanned (count <= 32)
+    int lo[3] = {ii[0], jj[0], kk[0]}, hi[3] = {ii[0], jj[0], kk[0]};
 #pragma unroll
     for (int u = 0; u < V; u++) {
-        vx[u] = (float)ii[u] - org.x;  // exact
-        vy[u] = (float)jj[u] - org.y;
-        vz[u] = (float)kk[u] - org.z;
-        vv[u] = vx[u] * vx[u] + vy[u] * vy[u] + vz[u] * vz[u];  // exact (integers below 2^24)
-        A2[u] = pack2(-2.f * vx[u], -2.f * vx[u]);
-        B2[u] = pack2(-2.f * vy[u], -2.f * vy[u]);
-        C2[u] = pack2(-2.f * vz[u], -2.f * vz[u]);
+        const float x = -2.f * ((float)ii[u] - org.x), y = -2.f * ((float)jj[u] - org.y),
+                    z = -2.f * ((float)kk[u] - org.z);  // exact
+        ax[u] = pack2(x, x);
+        ay[u] = pack2(y, y);
+        az[u] = pack2(z, z);
         best[u] = second[u] = kInf;
-        beste[u] = -1;
+        bestc[u] = -1;
         band[u] = 0u;
+        lo[0] = min(lo[0], ii[u]); hi[0] = max(hi[0], ii[u]);
+        lo[1] = min(lo[1], jj[u]); hi[1] = max(hi[1], jj[u]);
+        lo[2] = min(lo[2], kk[u]); hi[2] = max(hi[2], kk[u]);
     }
-    const float eps = 0.5f * eps2;
-    for (int c = count - 1; c >= 0; c--) {
-        const int e = S.pairs[first + c];
-        if (e >= ne) {
-            if ((threadIdx.x & 31) == 0) atomicOr(err, ERR_BOUNDS);
-            continue;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        lo[q] = __reduce_min_sync(kFull, lo[q]);
+        hi[q] = __reduce_max_sync(kFull, hi[q]);
+    }
+    // the centre (integers and halves: exact) and twice the half extents
+    const float cx = 0.5f * (float)(lo[0] + hi[0]) - org.x, cy = 0.5f * (float)(lo[1] + hi[1]) - org.y,
+                cz = 0.5f * (float)(lo[2] + hi[2]) - org.z;
+    const float Dx = (float)(hi[0] - lo[0]), Dy = (float)(hi[1] - lo[1]), Dz = (float)(hi[2] - lo[2]);
+    const float bx = -2.f * cx, by = -2.f * cy, bz = -2.f * cz, cc = cx * cx + cy * cy + cz * cz;
+    const float margin = 6.f * eps2;
+
+    float q0 = kInf, x0 = 0.f, y0 = 0.f, z0 = 0.f;
+    if (const int e0 = count > 0 ? S.pairs[first + count - 1] : ne; e0 < ne) {
+        const int2 r = S.erun[e0];
+        for (int t = lane; t < r.y; t += 32) {
+            const float4 p = pts[r.x + t];
+            const float q = qval(p, bx, by, bz);
+            if (q < q0) { q0 = q; x0 = p.x; y0 = p.y; z0 = p.z; }
         }
-        // skipped when no voxel can come within the band of its best through the
-        // element's box (best = kInf: never skipped)
-        const float* bx = S.box[e];
-        const float lx = bx[0], ly = bx[1], lz = bx[2], hx = bx[3], hy = bx[4], hz = bx[5];
-        bool need = false;
+        const int key = order_key(q0), least = __reduce_min_sync(kFull, key);
+        const int src = __ffs(__ballot_sync(kFull, key == least)) - 1;
+        q0 = __shfl_sync(kFull, q0, src);
+        x0 = __shfl_sync(kFull, x0, src);
+        y0 = __shfl_sync(kFull, y0, src);
+        z0 = __shfl_sync(kFull, z0, src);
+    }
+    const float limit = q0 + margin;
+    int ns = 0, ng = 0;
+    // the voxels against the buffered barycenters, two of them a packed FMA chain with the
+    // same three roundings each as qval; per group its least q, then per voxel the best and
+    // its element, and the least of the other elements
+    auto scan = [&]() {
+        __syncwarp();
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(W.f);  // 2 per pair
+        int i = 0;
+        for (int k = 0; k < ng; k++) {
+            const int c = W.cand[k], end = W.end[k];
+            float m[V];
 #pragma unroll
-        for (int u = 0; u < V; u++)
-            need = need || (active[u] && box_bound(vx[u], vy[u], vz[u], vv[u], lx, ly, lz, hx, hy, hz, eps) <=
-                                             best[u] + eps2);
-        if (!__any_sync(kFull, need)) continue;
-        const int2 r = S.erun[e];
-        float m[V];
-        run_min<V>(pts, r.x, r.y, A2, B2, C2, m);
+            for (int u = 0; u < V; u++) m[u] = kInf;
+#pragma unroll 2
+            for (; i < end; i += 2) {
+                const ulonglong2 xy = p[i], zw = p[i + 1];
 #pragma unroll
-        for (int u = 0; u < V; u++) {
-            if (m[u] < best[u]) {
-                second[u] = best[u];
-                best[u] = m[u];
-                beste[u] = e;
-            } else {
-                second[u] = fminf(second[u], m[u]);
+                for (int u = 0; u < V; u++)
+                    m[u] = min_of(m[u], fma2(az[u], zw.x, fma2(ay[u], xy.y, fma2(ax[u], xy.x, zw.y))));
             }
-            if (m[u] <= best[u] + eps2) band[u] |= 1u << (c & 31);
+#pragma unroll
+            for (int u = 0; u < V; u++) {
+                const bool same = c == bestc[u], less = m[u] < best[u];
+                second[u] = same ? second[u] : fminf(second[u], less ? best[u] : m[u]);
+                best[u] = fminf(best[u], m[u]);
+                bestc[u] = less ? c : bestc[u];
+                if (m[u] <= best[u] + eps2) band[u] |= 1u << (c & 31);
+            }
+        }
+        __syncwarp();
+        ns = ng = 0;
+    };
+    int g0 = 0;  // the open group's first entry
+    auto close = [&](int c) {
+        if (ns > g0) {
+            if (ns & 1) {
+                if (lane < 4) W.f[4 * (ns - 1) + 1 + 2 * lane] = lane == 3 ? kPadQ : 0.f;
+                ns++;
+            }
+            if (lane == 0) {
+                W.cand[ng] = (unsigned short)c;
+                W.end[ng] = (unsigned short)ns;
+            }
+            ng++;
+        }
+        g0 = ns;
+    };
+    for (int c0 = 0; c0 < count; c0 += 32) {
+        int2 run = make_int2(0, 0);
+        bool keep = false;
+        if (c0 + lane < count) {
+            const int e = S.pairs[first + c0 + lane];
+            if (e >= ne) {
+                atomicOr(err, ERR_BOUNDS);
+            } else {
+                const float* b = S.box[e];
+                const float dx = fmaxf(0.f, fmaxf(b[0] - cx, cx - b[3])), dy = fmaxf(0.f, fmaxf(b[1] - cy, cy - b[4])),
+                            dz = fmaxf(0.f, fmaxf(b[2] - cz, cz - b[5]));
+                const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                const float far = Dx * fmaxf(fabsf(b[0] - x0), fabsf(b[3] - x0)) +
+                                  Dy * fmaxf(fabsf(b[1] - y0), fabsf(b[4] - y0)) +
+                                  Dz * fmaxf(fabsf(b[2] - z0), fabsf(b[5] - z0));
+                // |c - box|^2 - |c|^2 against q_c(p0): a lower bound of q_c over the element
+                keep = !(d2 - cc > limit + far);
+                run = S.erun[e];
+            }
+        }
+        for (unsigned m = __ballot_sync(kFull, keep); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const int rx = __shfl_sync(kFull, run.x, l), ry = __shfl_sync(kFull, run.y, l);
+            for (int t0 = 0; t0 < ry; t0 += 32) {
+                const float4 p = pts[rx + min(t0 + lane, ry - 1)];
+                const float q = qval(p, bx, by, bz);
+                const bool can = t0 + lane < ry &&
+                                 q <= limit + (Dx * fabsf(p.x - x0) + Dy * fabsf(p.y - y0) + Dz * fabsf(p.z - z0));
+                const unsigned bal = __ballot_sync(kFull, can);
+                const int n = __popc(bal);
+                if (ns + n >= kSurv) {  // room for a padding entry too
+                    close(c0 + l);
+                    scan();
+                    g0 = 0;
+                }
+                if (can) {
+                    const int at = ns + __popc(bal & ((1u << lane) - 1));
+                    float* w = W.f + 8 * (at >> 1) + (at & 1);
+                    w[0] = p.x;
+                    w[2] = p.y;
+                    w[4] = p.z;
+                    w[6] = p.w;
+                }
+                ns += n;
+            }
+            close(c0 + l);
         }
     }
+    scan();
+    int beste[V];
+#pragma unroll
+    for (int u = 0; u < V; u++) beste[u] = bestc[u] >= 0 ? S.pairs[first + bestc[u]] : -1;
     // proven when every other element is farther by more than the band; a few near ties
     // are settled one voxel at a time by the whole warp, many by each lane for its own
     unsigned tie[V];
@@ -1312,7 +1391,6 @@ __device__ __forceinline__ void search_packet(const CorrSmem& S, const float4* p
         nties += __popc(tie[u]);
     }
     if (nties == 0) return;
-    const int lane = threadIdx.x & 31;
     if (nties <= kWarpTies) {
 #pragma unroll
         for (int u = 0; u < V; u++)
@@ -1330,8 +1408,8 @@ __device__ __forceinline__ void search_packet(const CorrSmem& S, const float4* p
         for (int u = 0; u < V; u++)
             if ((tie[u] >> lane) & 1u)
                 win[u] = exact_winner(S, pts, first, count, ne, eidx, eb, (double)ii[u], (double)jj[u],
-                                      (double)kk[u], -2.f * vx[u], -2.f * vy[u], -2.f * vz[u], best[u] + eps2,
-                                      band[u]);
+                                      (double)kk[u], -2.f * ((float)ii[u] - org.x), -2.f * ((float)jj[u] - org.y),
+                                      -2.f * ((float)kk[u] - org.z), best[u] + eps2, band[u]);
     }
 }
 
@@ -1364,17 +1442,21 @@ __device__ __forceinline__ void correct_voxel(const CorrectionArgs<T>& a, const 
     *outp = (T)o;
 }
 
-// A CTA per grain: the grain's element index, element boxes and FP32 barycenters are
-// staged in shared memory once; then, pass by pass over runs of kCVox consecutive voxels
-// of the box, the band voxels are grouped by IDLocal neighbour (counting sort in shared
-// memory) and the warps take packets of 32 voxels of one neighbour.
+// A CTA takes work items, runs of consecutive box voxels of one grain: the grain's element
+// index, element boxes and FP32 barycenters are staged in shared memory; then,
+// pass by pass over kCVox voxels, the band voxels are grouped by IDLocal neighbour and the
+// warps take packets of kPacket voxels of one neighbour.  About half of its time is the
+// grouping, which waits on loads and shared-memory atomics (24 warps an SM, 47% of the issue
+// slots); it was measured with the next loads in flight, with one look-up and atomic per
+// neighbour of a warp's voxels, and with the convolved values loaded ahead: none was faster.
 template <typename T>
-__global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs<T> a) {
+__global__ void __launch_bounds__(kCThreads, 3) correction_kernel(const __grid_constant__ CorrectionArgs<T> a) {
     extern __shared__ __align__(16) unsigned char corr_smem[];
     CorrSmem& S = *reinterpret_cast<CorrSmem*>(corr_smem);
     const double delta = a.geo.delta;
     const HullElements& el = a.el;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kCThreads / 32;
     const int n_items = a.item_off[a.G + 1];
     for (;;) {
         __syncthreads();  // the previous item's packets are done with the shared arrays
@@ -1384,7 +1466,7 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
         if (t >= n_items) break;
         const int pos = work_position(a.item_off, a.G, t);
         const int g = a.order[pos];
-        const long long item = t - a.item_off[pos];  // the run of box voxels this CTA takes
+        const int item = t - a.item_off[pos];  // the run of box voxels this CTA takes
         if (g < 1 || g > a.G) {
             if (threadIdx.x == 0) atomicOr(a.err, ERR_BOUNDS);
             continue;
@@ -1399,15 +1481,15 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
         const int npairs = min(el.pair_cap, kSPairs);
         const float4 org = el.eorg[g];
         const float4* gpts = el.ebf + (long long)g * el.flat_cap;
-        for (int q = threadIdx.x; q < kCHash; q += blockDim.x) S.hkey[q] = kNoId;
+        for (int q = threadIdx.x; q < kCHash; q += kCThreads) S.hkey[q] = kNoId;
         {  // the pair lists and the barycenters, copied asynchronously (waited for below)
             const uint4* src = reinterpret_cast<const uint4*>(el.idx_elem + (long long)g * el.pair_cap);
             uint4* dst = reinterpret_cast<uint4*>(S.pairs);
-            for (int q = threadIdx.x; q < npairs / 8; q += blockDim.x) cp_async16(dst + q, src + q);
+            for (int q = threadIdx.x; q < npairs / 8; q += kCThreads) cp_async16(dst + q, src + q);
             if (nflat <= kSPts)
-                for (int q = threadIdx.x; q < nflat; q += blockDim.x) cp_async16(S.pts + q, gpts + q);
+                for (int q = threadIdx.x; q < nflat; q += kCThreads) cp_async16(S.pts + q, gpts + q);
         }
-        for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+        for (int e = threadIdx.x; e < ne; e += kCThreads) {
             const HullElem& E = el.elem[(long long)g * el.elem_cap + e];
             int2 run = make_int2(E.pbase, E.pcount + (E.pcount & 1));  // with its padding entry
             if (run.x < 0 || (run.x & 1) || run.y < 0 || run.x + run.y > nflat) {
@@ -1424,7 +1506,7 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
         }
         cp_async_wait_all();
         __syncthreads();  // the hash is cleared, the copies have landed
-        for (int d = threadIdx.x; d < nd; d += blockDim.x) {
+        for (int d = threadIdx.x; d < nd; d += kCThreads) {
             const uint32_t id = el.idx_key[(long long)g * el.idx_cap + d];
             int2 r = el.idx_rng[(long long)g * el.idx_cap + d];
             if (r.x < 0 || r.y < 0 || r.x + r.y > npairs) {
@@ -1441,23 +1523,20 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                 hs = (hs + 1) & (kCHash - 1);
             }
         }
-        __syncthreads();
         const float4* pts = nflat <= kSPts ? S.pts : gpts;
+        __syncthreads();
         const int* eidx = el.eidx + (long long)g * el.flat_cap;
         const Box b = load_box(a.box + 6 * g);
-        const Box bo = load_box(a.idbox_old + 6 * g);
-        const long long old_count = bo.count();
+        const int old_count = (int)load_box(a.idbox_old + 6 * g).count();
         const T* in = a.in + a.in_off[g];
         T* out = a.out + a.out_off[g];
         const uint32_t* idl = a.id_old + a.idoff_old[g];
         const HullElem* elem = el.elem + (long long)g * el.elem_cap;
         const double* eb = el.ebary + 3 * (long long)g * el.bary_cap;
-        const int nx = b.nx(), ny = b.ny();
-        const int nxy = nx * ny;
-        const long long nvox = (long long)nxy * b.nz();
-        // a packet voxel's (z, y, x) from its flat index without 64-bit division
-        const bool fastdiv = nvox < (1LL << 24) && nx > 0;
-        const float rnxy = fastdiv ? __frcp_rn((float)nxy) : 0.f, rnx = fastdiv ? __frcp_rn((float)nx) : 0.f;
+        const int nx = b.nx(), nxy = nx * b.ny();
+        const int nvox = nxy * b.nz();  // below 2^24: sides are limited to a few hundred at most
+        // a packet voxel's (z, y, x) from its flat index without integer division
+        const float rnxy = __frcp_rn((float)nxy), rnx = __frcp_rn((float)nx);
         // the filter's error bound: q is within 16 R^2 2^-24 of |v' - p'|^2 - |v'|^2 (the
         // three FMAs, the FP32 rounding of p' and |p'|^2), R^2 the largest |v'|^2 or |p'|^2
         float r2 = org.w;
@@ -1470,22 +1549,21 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
         const float eps2 = fmaxf(2.f * 16.f * r2 * (1.0f / 16777216.f) * 1.0001f, 1e-6f);
         // passes over consecutive runs of kCVox voxels of the box, across rows and slices,
         // so that a pass holds many packets and few barriers are paid per voxel
-        const long long v_end = min(nvox, (item + 1) * kCItem);
-        for (long long v0 = item * kCItem; v0 < v_end; v0 += kCVox) {
-            const int nv = (int)min((long long)kCVox, v_end - v0);
-            for (int d = threadIdx.x; d < nd; d += blockDim.x) S.dcnt[d] = 0;
-            if (threadIdx.x == 0) S.pk_next = nwarps;  // packet w goes to warp w, the rest on demand
+        const int v_end = min(nvox, (item + 1) * a.item_vox);
+        for (int v0 = item * a.item_vox; v0 < v_end; v0 += kCVox) {
+            const int nv = min(kCVox, v_end - v0);
+            for (int d = threadIdx.x; d < nd; d += kCThreads) S.dcnt[d] = 0;
+            if (threadIdx.x == 0) S.pk_next = kWarps;  // packet w goes to warp w, the rest on demand
             __syncthreads();
             // band voxels: their neighbour; voxels whose neighbour no element holds get (1, 1)
             // now.  A batch of voxels per thread: their loads are in flight together.
             constexpr int kBatch = sizeof(T) == 4 ? 16 : 8;
-            for (int q0 = threadIdx.x; q0 < nv; q0 += kBatch * blockDim.x) {
+            for (int q0 = threadIdx.x; q0 < nv; q0 += kBatch * kCThreads) {
                 T vals[kBatch];
                 uint32_t ids[kBatch];
 #pragma unroll
                 for (int u = 0; u < kBatch; u++) {
-                    const int q = q0 + u * blockDim.x;
-                    const long long f = v0 + q;  // the box's flat [z][y][x] index
+                    const int q = q0 + u * kCThreads, f = v0 + q;
                     vals[u] = T(0);
                     ids[u] = 0u;
                     if (q < nv) {
@@ -1496,9 +1574,8 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                 }
 #pragma unroll
                 for (int u = 0; u < kBatch; u++) {
-                    const int q = q0 + u * blockDim.x;
+                    const int q = q0 + u * kCThreads;
                     if (q >= nv) continue;
-                    const long long fq = v0 + q;
                     unsigned short dd = kNoD;
                     if (fabs((double)vals[u]) < delta) {
                         const uint32_t id = ids[u];
@@ -1510,7 +1587,7 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                             hs = (hs + 1) & (kCHash - 1);
                         }
                         if (dd != kNoD) atomicAdd(&S.dcnt[dd], 1);
-                        else correct_voxel(a, elem, g, -1, id, (double)vals[u], (double)out[fq], out + fq);
+                        else correct_voxel(a, elem, g, -1, id, (double)vals[u], (double)out[v0 + q], out + (v0 + q));
                     }
                     S.vd[q] = dd;
                 }
@@ -1530,6 +1607,7 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                     if (d < nd) {
                         S.doff[d] = S.dcur[d] = run + ic - c;
                         S.dpk[d] = prun + ip - pk;
+                        for (int p = prun + ip - pk; p < prun + ip; p++) S.pkd[p] = (unsigned short)d;
                     }
                     run += __shfl_sync(kFull, ic, 31);
                     prun += __shfl_sync(kFull, ip, 31);
@@ -1537,43 +1615,30 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                 if (lane == 0) S.dpk[nd] = prun;
             }
             __syncthreads();
-            for (int q = threadIdx.x; q < nv; q += blockDim.x) {
-                const unsigned short dd = S.vd[q];
-                if (dd != kNoD) S.vlist[atomicAdd(&S.dcur[dd], 1)] = (unsigned short)q;
+            for (int q = threadIdx.x; q < nv; q += kCThreads) {
+                const unsigned d = S.vd[q];
+                if (d != kNoD) S.vlist[atomicAdd(&S.dcur[d], 1)] = (unsigned short)q;
             }
             __syncthreads();
             const int P = S.dpk[nd];
             for (int pk = warp; pk < P;) {
-                int lo = 0, hi = nd - 1;  // the neighbour whose packets hold pk
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (S.dpk[mid] <= pk) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int d = lo;
+                int nxt = 0;
+                if (lane == 0) nxt = atomicAdd(&S.pk_next, 1);  // the warp's next packet
+                const int d = S.pkd[pk];
                 const int start = S.doff[d] + (pk - S.dpk[d]) * kPacket;
                 const int cnt = min(kPacket, S.doff[d] + S.dcnt[d] - start);
                 bool active[kLV];
-                int ii[kLV], jj[kLV], kk[kLV], win[kLV];
-                long long f[kLV];
+                int ii[kLV], jj[kLV], kk[kLV], win[kLV], f[kLV];
                 T vin[kLV], vconv[kLV];
                 uint32_t id[kLV];
 #pragma unroll
                 for (int u = 0; u < kLV; u++) {
-                    const int slot = lane + 32 * u;
-                    active[u] = slot < cnt;
-                    const int q = S.vlist[start + (active[u] ? slot : 0)];
-                    f[u] = v0 + q;
+                    const int at = lane + 32 * u;
+                    active[u] = at < cnt;
+                    f[u] = v0 + S.vlist[start + (active[u] ? at : 0)];
                     int qz, rem, qy, qx;
-                    if (fastdiv) {
-                        divmod24((int)f[u], nxy, rnxy, qz, rem);
-                        divmod24(rem, nx, rnx, qy, qx);
-                    } else {
-                        qz = (int)(f[u] / nxy);
-                        rem = (int)(f[u] % nxy);
-                        qy = rem / nx;
-                        qx = rem % nx;
-                    }
+                    divmod24(f[u], nxy, rnxy, qz, rem);
+                    divmod24(rem, nx, rnx, qy, qx);
                     // the point is Vector3d(i, j, k), box.cpp:481
                     kk[u] = b.z0 + qz;
                     ii[u] = b.y0 + qy;
@@ -1585,16 +1650,15 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
                     if (active[u]) {
                         vin[u] = in[f[u]];
                         vconv[u] = out[f[u]];
-                        id[u] = f[u] < old_count ? idl[f[u]] : 0u;
+                        if (a.ph.use_see) id[u] = f[u] < old_count ? idl[f[u]] : 0u;
                     }
                 }
                 const int2 dr = S.drng[d];
-                search_packet<kLV>(S, pts, dr.x, dr.y, active, ii, jj, kk, org, eps2, ne, eidx, eb, a.err, win);
+                search_packet<kLV>(S, S.surv[warp], pts, dr.x, dr.y, active, ii, jj, kk, org, eps2, ne, eidx, eb,
+                                   a.err, win);
 #pragma unroll
                 for (int u = 0; u < kLV; u++)
                     if (active[u]) correct_voxel(a, elem, g, win[u], id[u], (double)vin[u], (double)vconv[u], out + f[u]);
-                int nxt = 0;
-                if (lane == 0) nxt = atomicAdd(&S.pk_next, 1);
                 pk = __shfl_sync(kFull, nxt, 0);
             }
             __syncthreads();
@@ -1605,7 +1669,13 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(CorrectionArgs
 }  // namespace
 
 size_t elements_scratch_per_cta() { return kElemScratch; }
-int correction_item_voxels() { return kCItem; }
+int correction_item_voxels(long long total, int num_sms) {
+    // A long run per item pays the staging once; below eight long runs per resident CTA (three
+    // an SM) single passes spread the work better: 30 grains of 90^3 voxels, one of which is
+    // up to 64 packets of one neighbour a pass, left three quarters of the warps idle with
+    // long runs (15.2 ms, against 7.6 with single passes and the same search).
+    return total >= 8LL * 3 * num_sms * kCItem ? kCItem : kCVox;
+}
 
 namespace {
 __global__ void faces_kernel(int G, const int* exists, HullElements el, const long long* off, int* count,

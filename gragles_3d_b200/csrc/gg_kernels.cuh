@@ -256,8 +256,7 @@ struct HullElements {
     // The same barycenters for the correction's FP32 filter, element by element in table
     // order (element e's at [pbase, pbase + pcount), pbase even, an odd run padded by one
     // entry with |p - o|^2 = 3e38): (p - o, |p - o|^2) in FP32, p - o and its square taken
-    // in FP64 first, with o the grain's integer origin.  Pairs of entries are interleaved
-    // as (x0, x1, y0, y1), (z0, z1, w0, w1) for the packed FMA.
+    // in FP64 first, with o the grain's integer origin.
     float4* ebf;              // (G + 1) x flat_cap
     int* eidx;                // (G + 1) x flat_cap: position of each of them in ebary (-1: padding)
     int* n_flat;              // G + 1: barycenters in ebf
@@ -322,9 +321,11 @@ struct CorrectionArgs {
     const int* order;         // grains by decreasing box (WorkOrder) and their work items,
     const int* item_off;      // fetched through *queue
     int* queue;
+    int item_vox;             // box voxels of an item
     int* err;
 };
-int correction_item_voxels();  // box voxels of one work item of the correction
+// Box voxels of one work item of the correction, for `total` voxels over all boxes.
+int correction_item_voxels(long long total, int num_sms);
 template <typename T>
 void launch_correction(const CorrectionArgs<T>& a, int grid, cudaStream_t s);
 

@@ -168,3 +168,35 @@ def test_correction_long_coarsening_stays_consistent(gpu):
         finals[prec] = trail[-1]
         gh.close()
     assert abs(finals[gpu.PRECISION_MIXED] - finals[gpu.PRECISION_FP64]) <= 0.01 * finals[gpu.PRECISION_FP64]
+
+
+def test_correction_of_large_hulls_matches_oracle(gpu, oracle):
+    """Three grains of a 44^3 domain, whose hulls have more barycenters than a CTA stages in
+    shared memory and more than a warp buffers for a packet (several buffers of candidates
+    per element): element counts exact, volumes to 1e-9 as above."""
+    n, g = 44, 3
+    ms = msgen.voronoi(n, g, seed=2144)
+    ms.euler[:] = np.array([[0.3, 0.5, 0.2], [0.38, 0.46, 0.25], [1.1, 0.9, 2.0]])
+    ext, counts = ms.grain_extents()
+    gh = gpu.GrainHandler(n, BORDER, 0.2, g, precision=gpu.PRECISION_FP64, correction=True, unique_energies=False,
+                          mobility_model=True)
+    gh.load(ms.labels, ext, counts)
+    gh.rtree_lists()
+    gh.set_orientations(ms.euler)
+    off = np.zeros(g + 2, np.int64)
+    ids = []
+    for i in range(1, g + 1):
+        ids.extend(gh.comparison_list(i).tolist())
+        off[i + 1] = len(ids)
+    osim = oracle.OracleSim(n, BORDER, 0.2, ms.labels, ext, counts, lists=(off, np.array(ids, np.uint32)))
+    osim.set_physics(True, unique_energies=False, mobility_model=True)
+    osim.set_orientations(ms.euler)
+    for s in range(3):
+        osim.step()
+        gh.step()
+        st = gh.stats()
+        for i in range(1, g + 1):
+            inf = osim.info(i)
+            assert bool(st.exists[i]) and inf["exists"], f"step {s} grain {i}"
+            assert gh.elements(i) == osim.elements(i), f"step {s} grain {i}: elements"
+            assert abs(st.volume[i] - inf["volume"]) <= 1e-9 * inf["volume"], f"step {s} grain {i}: volume"
