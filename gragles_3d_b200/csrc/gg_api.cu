@@ -676,7 +676,7 @@ int level_set_t(gg_ctx* ctx, int p, int regrid) {
     a.order = ctx->work.order;
     a.item_off = ctx->work.item_off;
     a.queue = ctx->work.queue;
-    launch_mc<T>(a, stage_grid(ctx, ST_LEVELSET), ctx->side_max, ctx->stream);
+    launch_mc<T>(a, stage_grid(ctx, ST_LEVELSET), ctx->side_max, ctx->grain_count, ctx->num_sms, ctx->stream);
     ctx->launches += 5;
     CK(cudaGetLastError());
     if (ctx->elements) {  // computeSurfaceElements, box.cpp:1175-1180

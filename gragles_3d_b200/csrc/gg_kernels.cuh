@@ -358,7 +358,7 @@ struct MCArgs {
     int* queue;
 };
 template <typename T>
-void launch_mc(const MCArgs<T>& a, int grid, int side, cudaStream_t s);
+void launch_mc(const MCArgs<T>& a, int grid, int side, int grains, int num_sms, cudaStream_t s);
 // Dynamic shared memory of the marching-cubes kernel for boxes up to `side`.
 size_t mc_slab_bytes(int side);
 

@@ -14,10 +14,12 @@
 // order, and processed further.  A block scan of per-cube triangle counts gives each
 // triangle its place in the reference's emission order; the FP64 volume and area
 // terms of a chunk are then added by one thread in that order, so the sums are
-// bit-identical to the reference's sequential loop.  The distinct neighbour IDs
+// bit-identical to the reference's sequential loop; the other warps go on meanwhile.  The distinct neighbour IDs
 // keep the reference's first-seen order through a shared-memory hash holding, per
 // ID, the smallest (cube index, rank in the cube's sorted list) key.
 #include "gg_kernels.cuh"
+
+#include <algorithm>
 
 namespace gg {
 
@@ -25,10 +27,8 @@ namespace gg {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kHash = 1024;  // distinct neighbour IDs per grain (power of two)
-static_assert(kThreads * 5 * sizeof(double) >= 2 * kHash * sizeof(unsigned), "ID collection aliases the volume buffer");
-constexpr int kSlabBytes = 36 * 1024;  // shared memory for a slab's sign bytes and cube lists
+constexpr int kSlabBytes = 36 * 1024;  // shared memory for a slab's sign bits and cube lists
+constexpr int kHash = 512;  // distinct neighbour IDs per grain (power of two, above the 256 kept)
 
 // cubeindex bit q <-> corner offset (dx, dy, dz), marchingCubes.cpp:376-385:
 // (0,0,1) (1,0,1) (1,0,0) (0,0,0) (0,1,1) (1,1,1) (1,1,0) (0,1,0); compile-time
@@ -104,8 +104,9 @@ __device__ __forceinline__ void hash_insert(unsigned* hkey, unsigned* hval, unsi
     atomicOr(err, ERR_NEIGHBORS);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 3) mc_kernel(MCArgs<T> a, int slab_bytes) {
+template <typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads, 768 / kThreads) mc_kernel(MCArgs<T> a, int slab_bytes) {
+    static_assert(kThreads * 5 * sizeof(double) >= 2 * kHash * sizeof(unsigned), "ID collection aliases the volume buffer");
     __shared__ double vbuf[kThreads * 5];
     __shared__ double abuf[kThreads * 5];
     __shared__ int warp_sums[33];
@@ -366,28 +367,41 @@ __global__ void __launch_bounds__(kThreads, 3) mc_kernel(MCArgs<T> a, int slab_b
                 }
             }
             __syncthreads();
-            if (threadIdx.x == 0) {  // in triangle order; eight terms' loads in flight at a time
-                int q = 0;
-                for (; q + 8 <= chunk_total; q += 8) {
-                    double tv[8], ta[8];
+            // The sums, in triangle order, by one thread with the next terms' loads ahead of the
+            // adds.  The other warps go on to the next cubes meanwhile: nothing overwrites the
+            // terms before that chunk's block scan, which this warp joins when it is done.
+            if (threadIdx.x == 0) {
+                constexpr int kAhead = 4;
+                double tv[kAhead], ta[kAhead];
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        tv[u] = vbuf[q + u];
-                        ta[u] = abuf[q + u];
+                for (int u = 0; u < kAhead; u++) {
+                    tv[u] = vbuf[u];  // past the chunk's terms: loaded, not added
+                    ta[u] = abuf[u];
+                }
+                int q = 0;
+                for (; q + kAhead <= chunk_total; q += kAhead) {
+                    double nv[kAhead], na[kAhead];
+#pragma unroll
+                    for (int u = 0; u < kAhead; u++) {
+                        nv[u] = vbuf[min(q + kAhead + u, 5 * kThreads - 1)];
+                        na[u] = abuf[min(q + kAhead + u, 5 * kThreads - 1)];
                     }
 #pragma unroll
-                    for (int u = 0; u < 8; u++) {
+                    for (int u = 0; u < kAhead; u++) {
+                        vol += tv[u];
+                        area += ta[u];
+                        tv[u] = nv[u];
+                        ta[u] = na[u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead - 1; u++)
+                    if (q + u < chunk_total) {
                         vol += tv[u];
                         area += ta[u];
                     }
-                }
-                for (; q < chunk_total; q++) {
-                    vol += vbuf[q];
-                    area += abuf[q];
-                }
             }
             ntri += chunk_total;
-            __syncthreads();
           }
           nrec += n_act;
         }
@@ -472,23 +486,38 @@ __global__ void count_kernel(int G, const int* present, const int* exists, const
 
 }  // namespace
 
-size_t mc_slab_bytes(int side) {
-    // at least one cube layer: two voxel layers of sign bits, the cube layer's active bits
-    // and a list entry per cube
+namespace {
+size_t layer_bytes(int side) {
+    // one cube layer: two voxel layers of sign bits, the cube layer's active bits and a list
+    // entry per cube
     const size_t n = side > 1 ? side : 2;
     const size_t pw = (n * n + 31) / 32, wr = (n - 1 + 31) / 32;
-    const size_t one_layer = 8 * pw + 16 + 4 * (n - 1) * wr + 2 * (n - 1) * (n - 1) + 4;
-    return one_layer > kSlabBytes ? one_layer : kSlabBytes;
+    return 8 * pw + 16 + 4 * (n - 1) * wr + 2 * (n - 1) * (n - 1) + 4;
 }
+}  // namespace
 
-template <typename T>
-void launch_mc(const MCArgs<T>& a, int grid, int side, cudaStream_t s) {
+size_t mc_slab_bytes(int side) { return std::max(layer_bytes(side), (size_t)kSlabBytes); }
+
+namespace {
+template <typename T, int kThreads>
+void launch_mc_threads(const MCArgs<T>& a, int grid, int side, cudaStream_t s) {
     static PerDevice configured;
     configured.once([] {
-        allow_max_dynamic_smem(mc_kernel<T>);
+        allow_max_dynamic_smem(mc_kernel<T, kThreads>);
     });
     const size_t bytes = mc_slab_bytes(side);
-    mc_kernel<T><<<grid, kThreads, bytes, s>>>(a, (int)bytes);
+    mc_kernel<T, kThreads><<<grid, kThreads, bytes, s>>>(a, (int)bytes);
+}
+}  // namespace
+
+template <typename T>
+void launch_mc(const MCArgs<T>& a, int grid, int side, int grains, int num_sms, cudaStream_t s) {
+    // A CTA takes a grain, so few grains leave SMs idle or with one CTA: then more threads a
+    // grain (level set 0.195 -> 0.152 ms at 20 grains with 512, 0.258 -> 0.205 ms at 200 with
+    // 384; at 2,000 and more the 256 of three CTAs an SM are the best, 0.55 against 0.63 ms).
+    if (grains <= num_sms) launch_mc_threads<T, 512>(a, grid, side, s);
+    else if (grains <= 2 * num_sms) launch_mc_threads<T, 384>(a, grid, side, s);
+    else launch_mc_threads<T, 256>(a, grid, side, s);
 }
 
 void launch_count(int G, const int* present, const int* exists, const int* box, int* out3, cudaStream_t s) {
@@ -496,7 +525,7 @@ void launch_count(int G, const int* present, const int* exists, const int* box, 
     count_kernel<<<64, 256, 0, s>>>(G, present, exists, box, out3);
 }
 
-template void launch_mc<double>(const MCArgs<double>&, int, int, cudaStream_t);
-template void launch_mc<float>(const MCArgs<float>&, int, int, cudaStream_t);
+template void launch_mc<double>(const MCArgs<double>&, int, int, int, int, cudaStream_t);
+template void launch_mc<float>(const MCArgs<float>&, int, int, int, int, cudaStream_t);
 
 }  // namespace gg

@@ -225,6 +225,27 @@ def test_comparison_of_ties_and_unlisted_neighbours_bitexact(gpu, oracle, border
                 assert np.array_equal(osim.sdf(g)[1], gh.sdf(g)[1]), f"step {s} grain {g}: field"
 
 
+@pytest.mark.parametrize("G", [40, 220, 420])
+def test_contour_at_every_cta_size_bitexact(gpu, oracle, G):
+    """The marching-cubes kernel's CTA size goes with the number of grains (few, some, many
+    against the SMs): volumes, surfaces and neighbours in first-seen order equal the oracle's."""
+    ms = msgen.voronoi(38, G, seed=3000 + G)
+    ext, counts = ms.grain_extents()
+    gh = gpu.GrainHandler(38, 5, 0.2, G, precision=0)
+    gh.load(ms.labels, ext, counts)
+    gh.default_lists()
+    osim = oracle.OracleSim(38, 5, 0.2, ms.labels, ext, counts, lists=_default_lists_from(gh))
+    for s in range(2):
+        assert gh.step()["grain_count"] == osim.step()
+    st = gh.stats()
+    for g in range(1, G + 1):
+        inf = osim.info(g)
+        assert bool(st.exists[g]) == inf["exists"], f"grain {g}"
+        if inf["exists"]:
+            assert st.volume[g] == inf["volume"] and st.surface[g] == inf["surface"], f"grain {g}"
+            assert np.array_equal(gh.neighbors(g), osim.neighbors(g)), f"grain {g}"
+
+
 def test_loop_mixed_volume_tolerance(gpu, oracle):
     c, gh, osim = _pair(gpu, oracle, "border10", precision=1)
     worst = 0.0
