@@ -90,6 +90,19 @@ def test_mixed_convolution_kernel_accuracy(gpu, oracle):
             assert err <= 4e-6, f"side {b.shape[0]}: relative max error {err:.3g}"
 
 
+@pytest.mark.parametrize("sides", [[65, 20], [95, 97, 1], [128, 33], [139]])
+def test_mixed_convolution_large_sides(gpu, oracle, sides):
+    """The FP32 kernels for sides above 64: one to five 32-wide column groups, row groups with
+    every remainder, smaller boxes in the same call, and the largest side, whose plane is
+    staged by halves; FP32-level error as above."""
+    rng = np.random.default_rng(18)
+    boxes = [rng.uniform(-0.1, 0.1, (n, n, n)).astype(np.float32) for n in sides]
+    for b, g in zip(boxes, gpu.convolve_boxes_mixed(boxes, 100, 0.2)):
+        want = oracle.convolve_box(b.astype(np.float64), 100, 0.2)
+        err = np.abs(g.astype(np.float64) - want).max() / np.abs(b).max()
+        assert err <= 4e-6, f"side {b.shape[0]}: relative max error {err:.3g}"
+
+
 def test_initial_sdf_bitexact(gpu, oracle):
     c, gh, osim = _pair(gpu, oracle, "tiny")
     for g in range(1, c["G"] + 1):
