@@ -40,6 +40,7 @@ struct gg_ctx {
     size_t esz = 8;
     Geometry geo{};
     cudaStream_t stream = nullptr;
+    SideStreams aux{};  // independent launches of one stage beside each other
     int num_sms = 148;
     int grid = 148 * 8;
     bool loaded = false;
@@ -338,12 +339,12 @@ int redistance(gg_ctx* ctx, int in_a, int out_a, const int* toff, int side, bool
     r.err = ctx->d_err;
     if (classes) {  // per size class of the output boxes (their tiles from toff)
         launch_redist_classes(ctx->G, toff, ctx->d_box[out_a], ctx->d_toff_rcls, ctx->stream);
-        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, ctx->d_toff_rcls, ctx->stream);
+        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, ctx->d_toff_rcls, &ctx->aux, ctx->stream);
         int nc = 0;
         for (int c = 0; c < kRedistClasses && (c == 0 || redist_side(c - 1) < side); c++) nc++;
         ctx->launches += 1 + 2 * nc;
     } else {
-        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, nullptr, ctx->stream);
+        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, nullptr, nullptr, ctx->stream);
         ctx->launches += 2;
     }
     CK(cudaGetLastError());
@@ -943,6 +944,11 @@ void free_all(gg_ctx* c) {
     if (c->h_total_vox) cudaFreeHost(c->h_total_vox);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
+    for (int i = 0; i < kSideStreams; i++) {
+        if (c->aux.stream[i]) cudaStreamDestroy(c->aux.stream[i]);
+        if (c->aux.join[i]) cudaEventDestroy(c->aux.join[i]);
+    }
+    if (c->aux.fork) cudaEventDestroy(c->aux.fork);
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
@@ -995,6 +1001,11 @@ int gg_create(const gg_params* params, gg_ctx** out) {
     CK(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, P.device));
     ctx->grid = ctx->num_sms * 8;
     for (auto& ev : ctx->ev) CK(cudaEventCreate(&ev));
+    for (int i = 0; i < kSideStreams; i++) {
+        CK(cudaStreamCreateWithFlags(&ctx->aux.stream[i], cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&ctx->aux.join[i], cudaEventDisableTiming));
+    }
+    CK(cudaEventCreateWithFlags(&ctx->aux.fork, cudaEventDisableTiming));
     const size_t G1 = (size_t)ctx->G + 1;
     CK(dalloc(&ctx->d_present, G1));
     CK(dalloc(&ctx->d_exists, G1));

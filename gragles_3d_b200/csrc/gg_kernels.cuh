@@ -429,9 +429,16 @@ __host__ __device__ constexpr int redist_units(int c) {
 }
 // class_toff: kRedistClasses tile tables of stride G + 2 (ceil(n / redist_units(c)) tiles
 // per grain of class c),
-// from launch_redist_classes; null: one launch over `a.toff` sized for `side`.
+// from launch_redist_classes; null: one launch over `a.toff` sized for `side`.  aux: the
+// context's own side streams, which wait for s and which s waits for (used with class_toff).
+constexpr int kSideStreams = 3;
+struct SideStreams {
+    cudaStream_t stream[kSideStreams];
+    cudaEvent_t fork, join[kSideStreams];
+};
 template <typename T>
-void launch_redistance(const RedistArgs<T>& a, int grid, int side, const int* class_toff, cudaStream_t s);
+void launch_redistance(const RedistArgs<T>& a, int grid, int side, const int* class_toff, const SideStreams* aux,
+                       cudaStream_t s);
 void launch_redist_classes(int G, const int* toff_all, const int* box, int* class_toff, cudaStream_t s);
 // Shared memory of one unit (one warp) at box side nmax; must fit one CTA.
 size_t redist_smem_bytes(int nmax, bool fp64);
