@@ -215,43 +215,41 @@ int put_table(gg_ctx* ctx, X** d, size_t* cap, const std::vector<X>& h) {
     return GG_OK;
 }
 
-// The tables of the current grid (N, M): DFT twiddles and the Gaussian multiplier per side,
-// and on the mixed path the circulant matrices.  Run at set-up and after a grid coarsening
-// (the Gaussian's dt N^2 is computed from the new N, grainhdl.cpp:1419-1442).
+// The tables of the current grid (N, M) for the sides a box can have: DFT twiddles and the
+// Gaussian multiplier per side on the FP64 path, the circulant matrices on the mixed path (as
+// the tensor-core operand up to its largest side, FP32 above).  Run at set-up and after a grid
+// coarsening (the Gaussian's dt N^2 is computed from the new N, grainhdl.cpp:1419-1442).
 int upload_tables(gg_ctx* ctx) {
-    const int M = ctx->M;
-    std::vector<double2> tw;
-    std::vector<long long> tw_off(M + 2, 0);
-    std::vector<double> gt;
-    std::vector<long long> g_off(M + 2, 0);
-    for (int n = 1; n <= M; n++) {
-        tw_off[n] = (long long)tw.size();
-        twiddle_table(n, tw);
-        g_off[n] = (long long)gt.size();
-        gaussian_table(n, ctx->N, ctx->P.time_step, gt);
-    }
-    int rc = put_table(ctx, &ctx->d_tw, &ctx->tw_cap, tw);
-    if (!rc) rc = put_table(ctx, &ctx->d_tw_off, &ctx->tw_off_cap, tw_off);
-    if (!rc) rc = put_table(ctx, &ctx->d_gtab, &ctx->gt_cap, gt);
-    if (!rc) rc = put_table(ctx, &ctx->d_g_off, &ctx->g_off_cap, g_off);
-    if (rc) return rc;
-    if (!ctx->fp64) {
+    const int M = ctx->M, top = std::min(M, ctx->side_limit);
+    int rc = GG_OK;
+    if (ctx->fp64) {
+        std::vector<double2> tw;
+        std::vector<long long> tw_off(M + 2, 0);
+        std::vector<double> gt;
+        std::vector<long long> g_off(M + 2, 0);
+        for (int n = 1; n <= top; n++) {
+            tw_off[n] = (long long)tw.size();
+            twiddle_table(n, tw);
+            g_off[n] = (long long)gt.size();
+            gaussian_table(n, ctx->N, ctx->P.time_step, gt);
+        }
+        rc = put_table(ctx, &ctx->d_tw, &ctx->tw_cap, tw);
+        if (!rc) rc = put_table(ctx, &ctx->d_tw_off, &ctx->tw_off_cap, tw_off);
+        if (!rc) rc = put_table(ctx, &ctx->d_gtab, &ctx->gt_cap, gt);
+        if (!rc) rc = put_table(ctx, &ctx->d_g_off, &ctx->g_off_cap, g_off);
+    } else {
         std::vector<float> circ;
         std::vector<long long> c_off(M + 2, 0);
-        for (int n = 1; n <= M; n++) {
-            c_off[n] = (long long)circ.size();
-            circulant_matrix(n, ctx->N, ctx->P.time_step, circ);
-        }
+        circulant_tables(ctx->N, ctx->P.time_step, kUmmaMaxSide + 1, top, nullptr, circ, c_off);
         rc = put_table(ctx, &ctx->d_circ, &ctx->circ_cap, circ);
         if (!rc) rc = put_table(ctx, &ctx->d_circ_off, &ctx->c_off_cap, c_off);
         std::vector<uint16_t> bmat;
         std::vector<long long> boff;
-        umma_tables(ctx->N, ctx->P.time_step, std::min(M, kUmmaMaxSide), bmat, boff);
+        umma_tables(ctx->N, ctx->P.time_step, std::min(top, kUmmaMaxSide), nullptr, bmat, boff);
         if (!rc) rc = put_table(ctx, &ctx->d_bmat, &ctx->bmat_cap, bmat);
         if (!rc) rc = put_table(ctx, &ctx->d_boff, &ctx->boff_cap, boff);
-        if (rc) return rc;
     }
-    return GG_OK;
+    return rc;
 }
 
 int check_err(gg_ctx* ctx, const char* where) {
@@ -1510,7 +1508,11 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     std::vector<double2> tw;
     std::vector<long long> tw_off(nmax + 2, 0), g_off(nmax + 2, 0);
     std::vector<double> gt;
+    std::vector<char> need(nmax + 1, 0);  // the tables of the sides there are
+    for (int b = 0; b < n_boxes; b++)
+        if (sides[b] >= 0) need[sides[b]] = 1;
     for (int n = 1; n <= nmax; n++) {
+        if (!need[n]) continue;
         tw_off[n] = (long long)tw.size();
         twiddle_table(n, tw);
         g_off[n] = (long long)gt.size();
@@ -1599,14 +1601,13 @@ int gg_convolve_boxes_mixed(const float* d_in, float* d_out, const int32_t* side
     std::vector<float> tab;
     std::vector<uint16_t> tab16;
     std::vector<long long> tab_off;
+    std::vector<char> need(nmax + 1, 0);  // the tables of the sides there are
+    for (int b = 0; b < n_boxes; b++) need[sides[b]] = 1;
     if (tc) {
-        umma_tables(domain_size, time_step, nmax, tab16, tab_off);
+        umma_tables(domain_size, time_step, nmax, &need, tab16, tab_off);
     } else {
         tab_off.assign(nmax + 2, 0);
-        for (int n = 1; n <= nmax; n++) {
-            tab_off[n] = (long long)tab.size();
-            circulant_matrix(n, domain_size, time_step, tab);
-        }
+        circulant_tables(domain_size, time_step, 1, nmax, &need, tab, tab_off);
     }
     float *d_tab = nullptr, *d_scr = nullptr;
     uint16_t* d_tab16 = nullptr;

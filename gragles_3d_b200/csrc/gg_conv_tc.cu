@@ -11,22 +11,37 @@
 
 namespace gg {
 
-void circulant_matrix(int n, int N, double time_step, std::vector<float>& out) {
+void circulant_matrix(int n, int N, double time_step, float* out) {
     // per-axis factor of box.cpp:760-761: exp(-sqrt(2/pi) 4 dt N^2 pi^2 / n^2 * f^2), f = min(k, n-k)
     const double pi = 3.14159265358979323846;
     const double dt = time_step / double(N * N);
     const double c = std::sqrt(2 / pi) * 4.0 * dt * double(N * N) / double(n * n) * pi * pi;
-    std::vector<long double> col(n);
+    std::vector<long double> factor(n);
+    for (int f = 0; f < n; f++) {
+        const int ff = f < n - f ? f : n - f;
+        factor[f] = std::exp(-(long double)c * ff * ff);
+    }
+    std::vector<float> col(n);
     for (int d = 0; d < n; d++) {
         long double acc = 0;
-        for (int f = 0; f < n; f++) {
-            const int ff = f < n - f ? f : n - f;
-            acc += std::exp(-(long double)c * ff * ff) * std::cos(2.0L * (long double)pi * f * d / n);
-        }
-        col[d] = acc / n;
+        for (int f = 0; f < n; f++) acc += factor[f] * std::cos(2.0L * (long double)pi * f * d / n);
+        col[d] = (float)(acc / n);
     }
     for (int p = 0; p < n; p++)
-        for (int q = 0; q < n; q++) out.push_back((float)col[(p - q + n) % n]);
+        for (int q = 0; q < n; q++) out[(size_t)p * n + q] = col[(p - q + n) % n];
+}
+
+void circulant_tables(int N, double time_step, int lo, int hi, const std::vector<char>* need, std::vector<float>& out,
+                      std::vector<long long>& off) {
+    long long total = 0;
+    for (int n = lo; n <= hi; n++) {
+        off[n] = total;
+        if (!need || (*need)[n]) total += (long long)n * n;
+    }
+    out.resize(total);
+    for_sides(lo, hi, [&](int n) {
+        if (!need || (*need)[n]) circulant_matrix(n, N, time_step, out.data() + off[n]);
+    });
 }
 
 namespace {

@@ -7,10 +7,40 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
+#include <new>
+#include <thread>
 #include <vector>
 
 namespace gg {
+
+// f(n) for every n in [lo, hi], the largest first, on up to 16 host threads.  The tables of one
+// side do not depend on another's, so who computes them does not matter; where no thread can be
+// started the caller does them all.  Throws when f has thrown.
+template <typename F>
+void for_sides(int lo, int hi, F&& f) {
+    std::atomic<int> next{hi};
+    std::atomic<bool> failed{false};
+    auto work = [&] {
+        try {
+            for (int n = next.fetch_sub(1); n >= lo; n = next.fetch_sub(1)) f(n);
+        } catch (...) {
+            failed = true;
+        }
+    };
+    std::vector<std::thread> threads;
+    const int count = std::min({(int)std::thread::hardware_concurrency(), 16, hi - lo + 1});
+    // below side 24 or so a thread costs more than all of the tables
+    if (hi >= 24) try {
+        for (int i = 1; i < count; i++) threads.emplace_back(work);
+    } catch (...) {
+    }
+    work();
+    for (auto& t : threads) t.join();
+    if (failed) throw std::bad_alloc();  // the only thing the tables can fail by
+}
 
 struct ConvTCArgs {
     int G;
@@ -25,8 +55,12 @@ struct ConvTCArgs {
     int* err;
 };
 
-// Append C_n (row-major, FP32) for box side n, domain size N and TimeStepSize.
-void circulant_matrix(int n, int N, double time_step, std::vector<float>& out);
+// Write C_n (row-major, FP32, n x n) for box side n, domain size N and TimeStepSize.
+void circulant_matrix(int n, int N, double time_step, float* out);
+// C_n of the sides lo..hi (those with need[n], when need is given) one after the other in
+// `out`, side n at off[n] (off sized hi + 2 or more by the caller).
+void circulant_tables(int N, double time_step, int lo, int hi, const std::vector<char>* need, std::vector<float>& out,
+                      std::vector<long long>& off);
 
 // toff holds n tiles per grain (z-planes, then y-rows).
 void launch_conv_tc(const ConvTCArgs& a, int num_sms, int side_max, cudaStream_t s);
@@ -68,8 +102,10 @@ struct UmmaConvArgs {
 int umma_side_limit();
 // True when the tensor-core kernel takes boxes up to side_max (else the SIMT kernels).
 bool umma_supported(int side_max);
-// C_n of every side 1..nmax as the MMA's B operand (hi block, then lo block).
-void umma_tables(int N, double time_step, int nmax, std::vector<uint16_t>& bmat, std::vector<long long>& boff);
+// C_n of every side 1..nmax (those with need[n], when need is given) as the MMA's B operand (hi
+// block, then lo block).
+void umma_tables(int N, double time_step, int nmax, const std::vector<char>* need, std::vector<uint16_t>& bmat,
+                 std::vector<long long>& boff);
 void launch_conv_umma(const UmmaConvArgs& a, int num_sms, int side_max, cudaStream_t s);
 
 }  // namespace gg

@@ -470,15 +470,21 @@ int umma_side_limit() { return kUmmaMaxSide; }
 
 bool umma_supported(int side_max) { return side_max >= 1 && side_max <= kUmmaMaxSide && umma_shape(side_max).R >= 2; }
 
-void umma_tables(int N, double time_step, int nmax, std::vector<uint16_t>& bmat, std::vector<long long>& boff) {
+void umma_tables(int N, double time_step, int nmax, const std::vector<char>* need, std::vector<uint16_t>& bmat,
+                 std::vector<long long>& boff) {
     boff.assign(nmax + 2, 0);
+    long long total = 0;
     for (int n = 1; n <= nmax; n++) {
-        std::vector<float> C;
-        circulant_matrix(n, N, time_step, C);
+        boff[n] = total;
+        if (!need || (*need)[n]) total += 2LL * round_n(n) * round_k(n);
+    }
+    bmat.assign(total, 0);
+    for_sides(1, nmax, [&](int n) {
+        if (need && !(*need)[n]) return;
+        std::vector<float> C((size_t)n * n);
+        circulant_matrix(n, N, time_step, C.data());
         const int kp = round_k(n), np = round_n(n), KC = kp / 8;
-        const size_t base = bmat.size();
-        boff[n] = (long long)base;
-        bmat.resize(base + 2 * (size_t)np * kp, 0);
+        const size_t base = boff[n];
         for (int r = 0; r < n; r++)
             for (int k = 0; k < n; k++) {
                 // B[k][r] = C[r][k] as the N x K K-major operand (row r = output column)
@@ -488,7 +494,7 @@ void umma_tables(int N, double time_step, int nmax, std::vector<uint16_t>& bmat,
                 bmat[base + pos] = __half_as_ushort(h);
                 bmat[base + (size_t)np * kp + pos] = __half_as_ushort(l);
             }
-    }
+    });
 }
 
 void launch_conv_umma(const UmmaConvArgs& c, int num_sms, int side_max, cudaStream_t s) {
