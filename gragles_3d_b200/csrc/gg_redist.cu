@@ -211,38 +211,315 @@ __device__ __forceinline__ void sweep_backward_in(T* o, int so, int d, int p_sta
     *op = cur;
 }
 
-// Shared-memory layout of a fixed-pitch class of largest side S (even, a multiple of 8):
-// one unit's output plane and input plane of S rows of pitch S + 1 (xy) or S x S (z),
-// units spaced so that lane t of the CTA, unit t / S, line t % S, reads bank t mod 32 in
-// every sweep (the unit stride is congruent to S modulo 32, as S (S + 1) is).
-__host__ __device__ constexpr int xy_unit_stride(int S) { return 2 * S * (S + 1) + (32 - S % 32) % 32; }
-static_assert(xy_unit_stride(24) % 4 == 0 && xy_unit_stride(40) % 4 == 0 && xy_unit_stride(56) % 4 == 0,
-              "unit planes start on 16 bytes");
-__host__ __device__ constexpr int z_unit_stride(int S) { return 2 * S * S + S % 32; }
+// ---- fixed-pitch classes (sides up to 64) ---------------------------------------------------
+// A thread runs its line's forward and backward sweep one after the other, so what the backward
+// sweep needs of the input is what the forward one saw: per position the sign, and per pair of
+// neighbours whether the product is <= 0, as 64-bit masks in registers.  So one shared plane per
+// slice (row) is enough: the x sweeps replace the staged input by the output in place, the y
+// and z sweeps read their input from global memory (adjacent threads, adjacent words, a group
+// ahead), and the backward sweep of y and z writes the result straight to global memory.
+struct LineSigns {
+    unsigned long long pos = 0, neg = 0, cross = 0;  // cross: bit p for the pair (p, p + 1)
+    template <typename T>
+    __device__ __forceinline__ void add(int p, T v) {
+        pos |= (unsigned long long)(v > T(0)) << p;
+        neg |= (unsigned long long)(v < T(0)) << p;
+    }
+    template <typename T>
+    __device__ __forceinline__ T step(int p, T h) const {  // isgn(in[p]) * h
+        return (pos >> p) & 1 ? h : ((neg >> p) & 1 ? -h : T(0));
+    }
+};
+
+// Bounds of a line's sweeps, positions relative to the output box (extent n): forward steps
+// p -> p + 1 for p0 <= p < pe, with the input (step_in) below pn, with the output's own sign
+// from there on; backward steps p -> p - 1 for ps >= p > 0, with the input above pm.
+// [lo, hi): the intersection along the line; inside: the line lies in the input across it.
+struct LineBounds {
+    int p0, pe, pn, ps, pm;
+    __device__ LineBounds(int lo, int hi, int n, bool inside) {
+        p0 = lo;
+        pe = n - 1;
+        pn = inside ? max(min(hi - 1, n - 1), lo) : lo;
+        ps = hi - 1;
+        pm = inside && ps > lo ? lo : ps;
+    }
+};
+
+// The interpolation of step_in at a sign change between a (here) and b.
+template <typename T>
+__device__ __forceinline__ void zero_cross(T a, T b, T& here, T h) {
+    const T slope = (b - a) / h;
+    const T dist = -a / slope;
+    if (fabs(here) > fabs(dist)) here = -dist * isgn(slope);
+}
+
+// The forward sweep (box.cpp:2367-2401, 2437-2472, 2501-2538): in(p), old(p) = the output
+// before it, put(p, v) = after it, in order of p.  Four steps at a time with the next four's
+// loads ahead; four without a sign change propagate with one sign.
+template <typename T, typename IN, typename OLD, typename PUT>
+__device__ __forceinline__ void forward_line(const LineBounds& L, T h, LineSigns& m, IN&& in, OLD&& old, PUT&& put) {
+    int p = L.p0;
+    if (p > L.pe) return;
+    T cur = old(p);
+    if (p < L.pn) {
+        T a = in(p), nb[4], nx[4];
+        m.add(p, a);
+        auto load = [&](int q) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                nb[j] = in(q + 1 + j);
+                nx[j] = old(q + 1 + j);
+            }
+        };
+        if (p + 4 <= L.pn) load(p);
+        for (; p + 4 <= L.pn; p += 4) {
+            T b[4], o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                b[j] = nb[j];
+                o[j] = nx[j];
+            }
+            if (p + 8 <= L.pn) load(p + 4);
+            const bool change = (a * b[0] <= T(0)) | (b[0] * b[1] <= T(0)) | (b[1] * b[2] <= T(0)) |
+                                (b[2] * b[3] <= T(0));
+            if (change) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const T from = j ? b[j - 1] : a;
+                    if (from * b[j] <= T(0)) {
+                        m.cross |= 1ull << (p + j);
+                        zero_cross(from, b[j], cur, h);
+                    }
+                    m.add(p + 1 + j, b[j]);
+                    step_prop(b[j], cur, o[j], h);
+                    put(p + j, cur);
+                    cur = o[j];
+                }
+            } else {
+                // a * b > 0 at every step: a and the four b share one sign and none is 0
+                const T inc = copysign_t(h, a);
+                const unsigned long long four = 0xFull << (p + 1);
+                if (a > T(0)) m.pos |= four;
+                else m.neg |= four;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const T cand = cur + inc;
+                    if (fabs(cand) < fabs(o[j])) o[j] = cand;
+                    put(p + j, cur);
+                    cur = o[j];
+                }
+            }
+            a = b[3];
+        }
+        for (; p < L.pn; p++) {
+            const T b = in(p + 1);
+            T o = old(p + 1);
+            if (a * b <= T(0)) {
+                m.cross |= 1ull << p;
+                zero_cross(a, b, cur, h);
+            }
+            m.add(p + 1, b);
+            step_prop(b, cur, o, h);
+            put(p, cur);
+            cur = o;
+            a = b;
+        }
+    }
+    for (; p < L.pe; p++) {
+        T o = old(p + 1);
+        step_prop(o, cur, o, h);
+        put(p, cur);
+        cur = o;
+    }
+    put(p, cur);
+}
+
+// The backward sweep from ps down to 0 (box.cpp:2403-2435, 2474-2496 and, with CROSS, which
+// interpolates at the forward sweep's sign changes, 2539-2576); put(p, v) in falling order of p.
+template <typename T, bool CROSS, typename IN, typename OLD, typename PUT>
+__device__ __forceinline__ void backward_line(const LineBounds& L, T h, const LineSigns& m, IN&& in, OLD&& old,
+                                              PUT&& put) {
+    int p = L.ps;
+    if (p < 0) return;
+    T cur = old(p);
+    for (; p - 4 >= L.pm; p -= 4) {
+        T o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = old(p - 1 - j);
+        const unsigned pos = (unsigned)(m.pos >> (p - 4)) & 15u, neg = (unsigned)(m.neg >> (p - 4)) & 15u;
+        const bool one = (pos == 15u || neg == 15u) && !(CROSS && ((unsigned)(m.cross >> (p - 4)) & 15u));
+        if (one) {
+            const T inc = pos ? h : -h;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const T cand = cur + inc;
+                if (fabs(cand) < fabs(o[j])) o[j] = cand;
+                put(p - j, cur);
+                cur = o[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int q = p - 1 - j;
+                if (CROSS && ((m.cross >> q) & 1)) zero_cross(in(q + 1), in(q), cur, h);
+                const T cand = cur + m.step(q, h);
+                if (fabs(cand) < fabs(o[j])) o[j] = cand;
+                put(p - j, cur);
+                cur = o[j];
+            }
+        }
+    }
+    for (; p > L.pm; p--) {
+        T o = old(p - 1);
+        if (CROSS && ((m.cross >> (p - 1)) & 1)) zero_cross(in(p), in(p - 1), cur, h);
+        const T cand = cur + m.step(p - 1, h);
+        if (fabs(cand) < fabs(o)) o = cand;
+        put(p, cur);
+        cur = o;
+    }
+    for (; p > 0; p--) {
+        T o = old(p - 1);
+        step_prop(o, cur, o, h);
+        put(p, cur);
+        cur = o;
+    }
+    put(0, cur);
+}
+
+// Elements of one unit's plane: rows of pitch S + 1 (xy) or [z][x] of pitch S (z), spaced so
+// that lane t of the CTA (unit t / S, line t % S) reads bank t mod 32 in every sweep.
+__host__ __device__ constexpr int xy_unit_stride(int S) { return S * (S + 1); }
+__host__ __device__ constexpr int z_unit_stride(int S) { return S * S + S % 32; }
+static_assert(xy_unit_stride(24) % 32 == 24 && xy_unit_stride(40) % 32 == 8 && xy_unit_stride(56) % 32 == 24, "banks");
 __host__ __device__ constexpr int class_threads(int S, int U) { return S ? (U * S + 31) / 32 * 32 : kMaxThreads; }
 
-// Kernel xy: a CTA per (grain, U consecutive output z-slices); unit u of the CTA owns
-// slice ob.z0 + U * tile + u, its threads run its rows for the x sweeps and its columns
-// for the y sweeps.  S = 0: one unit of runtime pitch (sides above the fixed classes).
+// Kernel xy, fixed pitch: a CTA per (grain, U consecutive output z-slices); the threads of unit
+// u (slice ob.z0 + U * tile + u) run its rows for the x sweeps and its columns for the y sweeps.
 template <typename T, int S, int U>
-__global__ void __launch_bounds__(kMaxThreads) redist_xy_kernel(RedistArgs<T> a) {
+__global__ void __launch_bounds__(class_threads(S, U)) redist_xy_lines(RedistArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tid = threadIdx.x;
-    const int u = S ? tid / S : 0;
-    const int line = S ? tid - u * S : tid;
-    const int lstride = S ? S : blockDim.x;
+    const int u = threadIdx.x / S, line = threadIdx.x - u * S;
+    constexpr int P = S + 1;
+    T* O = reinterpret_cast<T*>(smem_raw) + (u < U ? u : 0) * xy_unit_stride(S);
     const T h = (T)a.geo.h;
     for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid(); w.next()) {
         const int g = w.g;
         const Box ob = a.out.grain_box(g);
         const Box ib = a.in.grain_box(g);
-        const int k = ob.z0 + w.local * U + u;
+        const Intersect I(ib, ob);
+        const int n = ob.nx(), ny = ob.ny(), z = w.local * U + u, k = ob.z0 + z, inx = ib.nx();
         const bool unit = u < U && k < ob.z1;
+        const bool sweeps = unit && k >= I.zmin && k < I.zmax - 1;  // else no xy sweep reaches this slice
+        const int x0 = I.xmin - ob.x0, x1 = I.xmax - ob.x0, y0 = I.ymin - ob.y0, y1 = I.ymax - ob.y0;
+        T* outg = a.out.grain_ptr(g) + (long long)z * n * ny;
+        const T* ing = a.in.grain_ptr(g);
+        if (sweeps) {
+            // the rows of the intersection as one flat range, x-adjacent threads on x-adjacent
+            // words: element q is row q / wd, column q % wd
+            const int wd = x1 - x0, m = (y1 - y0) * wd;
+            const float rwd = 1.f / (float)wd;
+            const T* src = ing + ib.at(I.ymin, I.xmin, k);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(O + y0 * P + x0);
+            for (int q = line; q < m; q += S) {
+                const int r = div_small<S>(q, wd, rwd), c = q - r * wd;
+                cp_async_to(dst + (uint32_t)(sizeof(T) * (r * P + c)), src + (r * inx + c));
+            }
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        if (sweeps && line < ny) {  // x: the output is -1 everywhere before
+            T* row = O + line * P;
+            if (line >= y0) {
+                const LineBounds L(x0, x1, n, line < y1);
+                LineSigns m;
+                for (int p = 0; p < x0; p++) row[p] = T(-1);
+                forward_line(L, h, m, [&](int p) { return row[p]; }, [&](int) { return T(-1); },
+                             [&](int p, T v) { row[p] = v; });
+                backward_line<T, false>(L, h, m, [&](int) { return T(0); }, [&](int p) { return row[p]; },
+                                        [&](int p, T v) { row[p] = v; });
+            } else {
+                for (int p = 0; p < n; p++) row[p] = T(-1);
+            }
+        }
+        __syncthreads();
+        if (unit && line < n) {  // y
+            T* col = O + line;
+            T* dst = outg + line;
+            if (sweeps && line >= x0) {
+                const bool inside = line < x1;
+                const LineBounds L(y0, y1, ny, inside);
+                LineSigns m;
+                const T* src = ing + ib.at(ob.y0, ob.x0 + line, k);
+                forward_line(L, h, m, [&](int p) { return src[p * inx]; }, [&](int p) { return col[p * P]; },
+                             [&](int p, T v) { col[p * P] = v; });
+                for (int p = ny - 1; p > L.ps; p--) dst[p * n] = col[p * P];
+                backward_line<T, false>(L, h, m, [&](int) { return T(0); }, [&](int p) { return col[p * P]; },
+                                        [&](int p, T v) { dst[p * n] = v; });
+            } else {
+                for (int p = 0; p < ny; p++) dst[p * n] = sweeps ? col[p * P] : T(-1);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Kernel z, fixed pitch: a CTA per (grain, U consecutive output y-rows), a thread per column;
+// each thread's column of the shared plane is its own, so there is no barrier.
+template <typename T, int S, int U>
+__global__ void __launch_bounds__(class_threads(S, U)) redist_z_lines(RedistArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int u = threadIdx.x / S, x = threadIdx.x - u * S;
+    T* Z = reinterpret_cast<T*>(smem_raw) + (u < U ? u : 0) * z_unit_stride(S) + x;  // Z[p * S]
+    const T h = (T)a.geo.h;
+    const T delta = (T)a.geo.delta;
+    // clampValues(-delta, delta), dimensionalBufferReal.h:44-57
+    auto clamp = [&](T v) { return v < -delta ? -delta : (v > delta ? delta : v); };
+    for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid(); w.next()) {
+        const int g = w.g;
+        const Box ob = a.out.grain_box(g);
+        const Box ib = a.in.grain_box(g);
+        const Intersect I(ib, ob);
+        const int n = ob.nx(), nz = ob.nz(), y = w.local * U + u, i = ob.y0 + y, j = ob.x0 + x;
+        if (u >= U || x >= n || i >= ob.y1) continue;
+        const int zs = n * ob.ny(), izs = ib.nx() * ib.ny();
+        T* out = a.out.grain_ptr(g) + (y * n + x);
+        if (i >= I.ymin && j >= I.xmin) {
+            const LineBounds L(I.zmin - ob.z0, I.zmax - ob.z0, nz, i < I.ymax && j < I.xmax);
+            LineSigns m;
+            const T* src = a.in.grain_ptr(g) + ib.at(i, j, ob.z0);
+            auto in = [&](int p) { return src[p * izs]; };
+            for (int p = 0; p < L.p0; p++) Z[p * S] = out[p * zs];
+            forward_line(L, h, m, in, [&](int p) { return out[p * zs]; }, [&](int p, T v) { Z[p * S] = v; });
+            for (int p = nz - 1; p > L.ps; p--) out[p * zs] = clamp(Z[p * S]);
+            backward_line<T, true>(L, h, m, in, [&](int p) { return Z[p * S]; },
+                                   [&](int p, T v) { out[p * zs] = clamp(v); });
+        } else {
+            for (int p = 0; p < nz; p++) out[p * zs] = clamp(out[p * zs]);
+        }
+    }
+}
+
+// ---- runtime pitch (the load's first redistancing, and sides above 64) ----------------------
+// Kernel xy: a CTA per (grain, output z-slice), the slice's output and input planes in shared
+// memory; its threads run its rows for the x sweeps and its columns for the y sweeps.
+template <typename T>
+__global__ void __launch_bounds__(kMaxThreads) redist_xy_kernel(RedistArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int tid = threadIdx.x;
+    const int line = tid, lstride = blockDim.x;
+    const T h = (T)a.geo.h;
+    for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid(); w.next()) {
+        const int g = w.g;
+        const Box ob = a.out.grain_box(g);
+        const Box ib = a.in.grain_box(g);
+        const int k = ob.z0 + w.local;
+        const bool unit = k < ob.z1;
         const Intersect I(ib, ob);
         const int nx = ob.nx(), ny = ob.ny();
-        const int P = S ? S + 1 : (nx | 1);
-        const int PL = S ? S * (S + 1) : ny * P;  // the input plane follows the output plane
-        T* O = reinterpret_cast<T*>(smem_raw) + (S ? u * xy_unit_stride(S) : 0);
+        const int P = nx | 1;
+        const int PL = ny * P;  // the input plane follows the output plane
+        T* O = reinterpret_cast<T*>(smem_raw);
         T* In = O + PL;
         T* outg = a.out.grain_ptr(g) + (long long)(k - ob.z0) * nx * ny;
         const bool sweeps = unit && k >= I.zmin && k < I.zmax - 1;
@@ -264,7 +541,7 @@ __global__ void __launch_bounds__(kMaxThreads) redist_xy_kernel(RedistArgs<T> a)
             const T* src = a.in.grain_ptr(g) + ib.at(I.ymin, I.xmin, k);
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(In + (I.ymin - ob.y0) * P + (I.xmin - ob.x0));
             for (int q = line; q < n; q += lstride) {
-                const int r = div_small<S>(q, wd, rwd), c = q - r * wd;
+                const int r = div_small<0>(q, wd, rwd), c = q - r * wd;
                 cp_async_to(dst + (uint32_t)(sizeof(T) * (r * P + c)), src + (r * inx + c));
             }
         }
@@ -291,7 +568,7 @@ __global__ void __launch_bounds__(kMaxThreads) redist_xy_kernel(RedistArgs<T> a)
         if (sweeps) {
             const float rnx = 1.f / (float)nx;
             for (int q = line; q < nx * ny; q += lstride) {
-                const int r = div_small<S>(q, nx, rnx);
+                const int r = div_small<0>(q, nx, rnx);
                 outg[q] = O[r * P + (q - r * nx)];
             }
         }
@@ -299,30 +576,27 @@ __global__ void __launch_bounds__(kMaxThreads) redist_xy_kernel(RedistArgs<T> a)
     }
 }
 
-// Kernel z: a CTA per (grain, U consecutive output y-rows); unit u owns row
-// ob.y0 + U * tile + u, whose [z][x] plane sits in shared memory, and its threads run
-// the z recurrences of one column each (x-adjacent threads touch adjacent words).
-template <typename T, int S, int U>
+// Kernel z: a CTA per (grain, output y-row), whose [z][x] planes sit in shared memory; its
+// threads run the z recurrences of one column each (x-adjacent threads touch adjacent words).
+template <typename T>
 __global__ void __launch_bounds__(kMaxThreads) redist_z_kernel(RedistArgs<T> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x;
-    const int u = S ? tid / S : 0;
-    const int line = S ? tid - u * S : tid;
-    const int lstride = S ? S : blockDim.x;
+    const int line = tid, lstride = blockDim.x;
     const T h = (T)a.geo.h;
     const T delta = (T)a.geo.delta;
     for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid(); w.next()) {
         const int g = w.g;
         const Box ob = a.out.grain_box(g);
         const Box ib = a.in.grain_box(g);
-        const int i = ob.y0 + w.local * U + u;
-        const bool unit = u < U && i < ob.y1;
+        const int i = ob.y0 + w.local;
+        const bool unit = i < ob.y1;
         const Intersect I(ib, ob);
         const int nx = ob.nx(), nz = ob.nz();
-        const int PZ = S ? S : nx;                // z stride in shared memory
-        const int PLZ = S ? S * S : nx * nz;      // the input plane follows the output plane
+        const int PZ = nx;        // z stride in shared memory
+        const int PLZ = nx * nz;  // the input plane follows the output plane
         const long long zs = (long long)nx * ob.ny();  // z stride of the output box
-        T* Z = reinterpret_cast<T*>(smem_raw) + (S ? u * z_unit_stride(S) : 0);
+        T* Z = reinterpret_cast<T*>(smem_raw);
         T* Zin = Z + PLZ;
         T* outr = a.out.grain_ptr(g) + (long long)(i - ob.y0) * nx;  // OUT(i, x0, z0)
         const float rnx = 1.f / (float)nx;
@@ -331,7 +605,7 @@ __global__ void __launch_bounds__(kMaxThreads) redist_z_kernel(RedistArgs<T> a) 
             // range (element q: z q / width, x q % width), x-adjacent threads on x-adjacent words
             const uint32_t zd = (uint32_t)__cvta_generic_to_shared(Z);
             for (int q = line; q < nz * nx; q += lstride) {
-                const int r = div_small<S>(q, nx, rnx), c = q - r * nx;
+                const int r = div_small<0>(q, nx, rnx), c = q - r * nx;
                 cp_async_to(zd + (uint32_t)(sizeof(T) * (r * PZ + c)), outr + (r * zs + c));
             }
             if (i >= I.ymin && i < I.ymax) {
@@ -341,7 +615,7 @@ __global__ void __launch_bounds__(kMaxThreads) redist_z_kernel(RedistArgs<T> a) 
                 const T* src = a.in.grain_ptr(g) + ib.at(i, I.xmin, I.zmin);
                 const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Zin + (I.zmin - ob.z0) * PZ + (I.xmin - ob.x0));
                 for (int q = line; q < n; q += lstride) {
-                    const int r = div_small<S>(q, wd, rwd), c = q - r * wd;
+                    const int r = div_small<0>(q, wd, rwd), c = q - r * wd;
                     cp_async_to(dst + (uint32_t)(sizeof(T) * (r * PZ + c)), src + (r * izs + c));
                 }
             }
@@ -362,7 +636,7 @@ __global__ void __launch_bounds__(kMaxThreads) redist_z_kernel(RedistArgs<T> a) 
         // clampValues(-delta, delta), dimensionalBufferReal.h:44-57
         if (unit)
             for (int q = line; q < nz * nx; q += lstride) {
-                const int r = div_small<S>(q, nx, rnx), c = q - r * nx;
+                const int r = div_small<0>(q, nx, rnx), c = q - r * nx;
                 T v = Z[r * PZ + c];
                 if (v < -delta) v = -delta;
                 else if (v > delta) v = delta;
@@ -466,23 +740,32 @@ void launch_redist_classes(int G, const int* toff_all, const int* box, int* clas
 namespace {
 template <typename T, int S, int U>
 void launch_class(const RedistArgs<T>& a, int n, cudaStream_t s) {
-    static_assert(S % 8 == 0 && U * S <= kMaxThreads, "fixed-pitch classes: sides a multiple of 8");
-    static PerDevice configured;
-    configured.once([] {
-        allow_max_dynamic_smem(redist_xy_kernel<T, S, U>);
-        allow_max_dynamic_smem(redist_z_kernel<T, S, U>);
-    });
-    const int threads = S ? class_threads(S, U) : std::min((n + 31) / 32 * 32, kMaxThreads);
     // Each CTA takes an equal share of the tiles; with one share per resident CTA the slots that
     // another class's launch frees late finish late.  Several shares a slot let the hardware even
     // that out: 8.25 -> 7.8 ms (256^3 / 20,000), 1.11 -> 0.95 (128^3 / 2,000); a few grains have
     // too few tiles for it.
     const int shares = std::min(8, std::max(1, a.G / 50));
-    const size_t e = sizeof(T);
-    const size_t sxy = S ? (size_t)U * xy_unit_stride(S) * e : redist_smem_bytes(n, e == 8);
-    const size_t sz = S ? (size_t)U * z_unit_stride(S) * e : redist_smem_bytes(n, e == 8);
-    redist_xy_kernel<T, S, U><<<shares * resident_ctas(redist_xy_kernel<T, S, U>, threads, sxy), threads, sxy, s>>>(a);
-    redist_z_kernel<T, S, U><<<shares * resident_ctas(redist_z_kernel<T, S, U>, threads, sz), threads, sz, s>>>(a);
+    static PerDevice configured;
+    if constexpr (S > 0) {
+        static_assert(S % 8 == 0 && S <= 64 && U * S <= kMaxThreads, "sides a multiple of 8, masks of 64 bits");
+        configured.once([] {
+            allow_max_dynamic_smem(redist_xy_lines<T, S, U>);
+            allow_max_dynamic_smem(redist_z_lines<T, S, U>);
+        });
+        const int threads = class_threads(S, U);
+        const size_t sxy = (size_t)U * xy_unit_stride(S) * sizeof(T), sz = (size_t)U * z_unit_stride(S) * sizeof(T);
+        redist_xy_lines<T, S, U><<<shares * resident_ctas(redist_xy_lines<T, S, U>, threads, sxy), threads, sxy, s>>>(a);
+        redist_z_lines<T, S, U><<<shares * resident_ctas(redist_z_lines<T, S, U>, threads, sz), threads, sz, s>>>(a);
+    } else {
+        configured.once([] {
+            allow_max_dynamic_smem(redist_xy_kernel<T>);
+            allow_max_dynamic_smem(redist_z_kernel<T>);
+        });
+        const int threads = std::min((n + 31) / 32 * 32, kMaxThreads);
+        const size_t smem = redist_smem_bytes(n, sizeof(T) == 8);
+        redist_xy_kernel<T><<<shares * resident_ctas(redist_xy_kernel<T>, threads, smem), threads, smem, s>>>(a);
+        redist_z_kernel<T><<<shares * resident_ctas(redist_z_kernel<T>, threads, smem), threads, smem, s>>>(a);
+    }
 }
 }  // namespace
 
@@ -492,14 +775,14 @@ void launch_redistance(const RedistArgs<T>& a, int grid, int side, const int* cl
     if (!class_toff) {  // one unit per CTA of runtime pitch, over a.toff (n tiles a grain)
         static PerDevice configured;
         configured.once([] {
-            allow_max_dynamic_smem(redist_xy_kernel<T, 0, 1>);
-            allow_max_dynamic_smem(redist_z_kernel<T, 0, 1>);
+            allow_max_dynamic_smem(redist_xy_kernel<T>);
+            allow_max_dynamic_smem(redist_z_kernel<T>);
         });
         const size_t smem = redist_smem_bytes(side, sizeof(T) == 8);
         int threads = (side + 31) / 32 * 32;
         threads = threads > kMaxThreads ? kMaxThreads : threads;
-        redist_xy_kernel<T, 0, 1><<<grid * 2, threads, smem, s>>>(a);
-        redist_z_kernel<T, 0, 1><<<grid * 2, threads, smem, s>>>(a);
+        redist_xy_kernel<T><<<grid * 2, threads, smem, s>>>(a);
+        redist_z_kernel<T><<<grid * 2, threads, smem, s>>>(a);
         return;
     }
     // One pair of launches per size class up to the largest side, each filling the device with
