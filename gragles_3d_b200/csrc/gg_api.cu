@@ -454,8 +454,8 @@ int stage_convolution_t(gg_ctx* ctx) {
         a.tw_off = ctx->d_tw_off;
         a.gtab = ctx->d_gtab;
         a.g_off = ctx->d_g_off;
-        launch_conv_f64(a, stage_grid(ctx, ST_CONV), ctx->side_max, ctx->stream);
-        ctx->launches += 3;
+        launch_conv_f64(a, ctx->side_max, ctx->stream);
+        ctx->launches += 5;
     } else {
         // two size classes in one step: sides up to kUmmaMaxSide on the tensor cores, larger
         // boxes (when any) on the FP32 SIMT kernels; each launch walks only its class's tiles
@@ -1501,9 +1501,6 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     if (!d_in || !d_out || !sides || !offs || n_boxes < 1 || domain_size < 1) return GG_ERR_INVALID;
     int nmax = 0;
     for (int b = 0; b < n_boxes; b++) nmax = std::max(nmax, (int)sides[b]);
-    int dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (nmax < 1 || nmax > kConvF64MaxSide) return GG_ERR_UNSUPPORTED;
     std::vector<double2> tw;
     std::vector<long long> tw_off(nmax + 2, 0), g_off(nmax + 2, 0);
@@ -1567,7 +1564,7 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     a.tw_off = d_tw_off;
     a.gtab = d_gt;
     a.g_off = d_g_off;
-    launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, nmax, 0);
+    launch_conv_f64(a, nmax, 0);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     void* ptrs[] = {d_tw, d_gt, d_tw_off, d_g_off, d_spec, d_box, d_off, d_spec_off, d_toff};

@@ -22,10 +22,10 @@ struct ConvArgs {
     const long long* g_off;
 };
 
-// Largest box side the FP64 convolution takes: a plane and two complex half-spectra of
-// it in 227 KB of shared memory.
+// Largest box side the FP64 convolution takes (a plane and two complex half-spectra of it
+// fill 227 KB of shared memory).
 constexpr int kConvF64MaxSide = 97;
-// nmax: the largest side among the boxes of the tiles.
-void launch_conv_f64(const ConvArgs& a, int grid, int nmax, cudaStream_t s);
+// Five launches; nmax: the largest side among the boxes of the tiles.
+void launch_conv_f64(const ConvArgs& a, int nmax, cudaStream_t s);
 
 }  // namespace gg

@@ -9,10 +9,12 @@
 // is one fma chain over m = 0..n-1 with twiddle index (k*m) mod n taken from a
 // host-built libm table, and G comes from a host-built table per box side.  These
 // kernels run exactly those chains, so the FP64 path is bit-identical to the
-// oracle.  The transform is split in three batched passes over all boxes:
-//   A  per (grain, z-plane): x r2c, then y                    -> spectrum scratch
-//   B  per 8 (ky, kx) lines: z forward, multiply by G, z inverse (in place)
-//   C  per (grain, z-plane): y inverse, then x c2r            -> output arena
+// oracle.  The transform runs in five batched passes over all boxes' lines:
+//   x forward (real to half spectrum) -> spectrum scratch; y forward, in place; z forward,
+//   multiply by G, z inverse, in place; y inverse, in place; x inverse -> output arena.
+// A warp takes 8 lines (16 rows in x) at a time: its lines, twiddles and products are its own,
+// so nothing waits on a block barrier, and lines are numbered through a whole box, so that
+// only a box's last fragment is part-full.
 //
 // A chain is a row of a product with the twiddle matrix: a complex output's real part is
 // sum over m of z.x w.x, then z.y w.y, a dot product of length 2n, and its imaginary part
@@ -23,14 +25,15 @@
 // measured for both); what it removes is everything around the arithmetic.  The scalar
 // form of these passes read a 16-byte twiddle and updated an index for every four fma and
 // left the lanes past a box's last line idle: 11.5 ms for the 2,000 boxes of a 128^3
-// domain (19% of the FP64 rate); this form takes 4.04 ms, its passes 59%, 73% and 52% of the matrix
-// pipe's cycles, the rest going to barriers, operand loads and the tails of fragments (at
-// n = 35 the frequencies fill 35 of 40 columns).  A step that pads a chain adds
-// (-0) x (+0) = -0, which leaves any accumulator as it is.
+// domain (19% of the FP64 rate).  With x and y of a plane in one block (three passes, less
+// traffic) the matrix pipe was 52-59% busy, waiting at barriers, and the passes took 4.0 ms;
+// these take 3.5 ms, the pipe 70-73% busy in y and z and 51% in x.  The frequencies still pad
+// (35 of 40 columns at n = 35).  A step that pads a chain adds (-0) x (+0) = -0, which leaves
+// any accumulator as it is.
 //
 // B operands come from the side's n twiddles in shared memory, at an index each lane
 // advances (one add and one conditional subtraction per fragment), not from a stored
-// matrix: 2 n^2 doubles would take 65 KB at n = 64 and leave no room for the planes.
+// matrix: 2 n^2 doubles would take 65 KB at n = 64 and leave no room for the lines.
 #include "gg_common.cuh"
 #include "gg_conv.cuh"
 
@@ -40,15 +43,12 @@ namespace gg {
 
 namespace {
 
-constexpr int kThreads = 192;      // passes A and C: a warp per column fragment of sides up to 48
+constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kThreadsB = 256;     // pass B (its warps are independent)
-constexpr int kLineChunk = 6;      // line fragments of a complex product held in registers at once
-constexpr int kRealChunk = 10;     // of a real one
-constexpr int kPlanes = 4;         // most planes a tile of passes A and C takes together
-constexpr int kTileBytes = 64 * 1024;  // shared memory of a tile of several planes: three CTAs an SM
-constexpr int kColChunk = 8;   // column fragments of a pass B product held in registers at once
-constexpr int kLP = 12;        // pitch of pass B's 8 lines
+constexpr int kColChunk = 8;   // column fragments of a product held in registers at once (8 lines)
+constexpr int kRowFrags = 2;   // fragments of 8 rows an x pass takes
+constexpr int kRowChunk = 4;   // column fragments of x forward held in registers at once (16 rows)
+constexpr int kLP = 12;        // pitch of 8 complex lines
 
 // Pitches in elements.  The 16 lanes of a half warp read 4 lines x (2 rows of m) x (x, y)
 // of a complex [m][line] buffer, or 4 lines x 4 m of a [line][m] one: 128 bytes on
@@ -147,365 +147,315 @@ __device__ __forceinline__ void dispatch(int v, F&& f) {
     f(Int<MAX>{});
 }
 
-// Complex DFT along the nl lines of a [m][line] plane in shared memory, one item per (8
-// frequencies, chunk of lines); rot carries the round robin over the warps from one step
-// to the next so that every scheduler gets the same share.  store(l, k, re, im).
-template <bool INV, typename F>
-__device__ __forceinline__ void cdft_plane(const double2* src, int sm, int n, int nl, const double2* tw, int& rot,
-                                           F&& store) {
-    const Lane L;
-    const int lf = (nl + 7) / 8, cf = (n + 7) / 8;
-    const int chunks = (lf + kLineChunk - 1) / kLineChunk, per = (lf + chunks - 1) / chunks;
-    const int items = cf * chunks;
-    for (int it = ((threadIdx.x >> 5) + kWarps - rot) % kWarps; it < items; it += kWarps) {
-        const int kf = it / chunks, l0 = (it - kf * chunks) * per;
-        __syncwarp();
-        dispatch<kLineChunk>(min(per, lf - l0), [&](auto mt) {
-            constexpr int MT = decltype(mt)::value;
-            double re[MT][1][2], im[MT][1][2];
-            cdft<INV, MT, 1>(reinterpret_cast<const double*>(src + l0 * 8), 2 * sm, n, kf,
-                             reinterpret_cast<const double*>(tw), L, re, im);
-#pragma unroll
-            for (int j = 0; j < MT; j++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int l = (l0 + j) * 8 + L.r, k = kf * 8 + 2 * L.q + e;
-                    if (l < nl && k < n) store(l, k, re[j][0][e], im[j][0][e]);
-                }
-        });
-    }
-    rot = (rot + items) % kWarps;
+__device__ __forceinline__ void load_twiddles(double2* tw_s, const double2* __restrict__ tw, int n, int lane) {
+    for (int j = lane; j < n; j += 32) tw_s[j] = tw[j];
 }
 
-// Real-input DFT (x axis, r2c) along the nl lines of a [line][m] plane: frequencies k < nk.
+// One warp's walk over the fragments of `per` lines of all boxes: calls f(g, n, twiddles,
+// buffer, first line, lines of the box).  A grain's n tiles share its fragments, two or three
+// each; with few tiles for the warps, four warps share a tile's.
 template <typename F>
-__device__ __forceinline__ void r2c_plane(const double* src, int sl, int n, int nl, int nk, const double2* tw, int& rot,
-                                          F&& store) {
-    const Lane L;
-    const int lf = (nl + 7) / 8, cf = (nk + 7) / 8;
-    const int chunks = lf > kLineChunk ? (lf + kLineChunk - 1) / kLineChunk : (lf > 1 ? 2 : 1);
-    const int per = (lf + chunks - 1) / chunks;
-    const int items = cf * chunks;
-    for (int it = ((threadIdx.x >> 5) + kWarps - rot) % kWarps; it < items; it += kWarps) {
-        const int kf = it / chunks, l0 = (it - kf * chunks) * per;
-        if (l0 >= lf) continue;
-        __syncwarp();
-        dispatch<kLineChunk>(min(per, lf - l0), [&](auto mt) {
-            constexpr int MT = decltype(mt)::value;
-            double re[MT][2], im[MT][2];
-#pragma unroll
-            for (int j = 0; j < MT; j++) re[j][0] = re[j][1] = im[j][0] = im[j][1] = 0.0;
-            const int k = (kf * 8 + L.r) % n;
-            int t = (L.q * k) % n;
-            const int inc = (4 * k) % n;
-            const double* s = src + (l0 * 8 + L.r) * sl + L.q;
-            auto step = [&](int keep) {
-                const double2 w = tw[t];
-                const double c = keep_or(w.x, keep, 0), d = keep_or(-w.y, keep, 0);
-                t += inc;
-                if (t >= n) t -= n;
-#pragma unroll
-                for (int j = 0; j < MT; j++) {
-                    const double x = keep_or(s[8 * j * sl], keep, 1);
-                    mma_f64(re[j], x, c);
-                    mma_f64(im[j], x, d);
-                }
-            };
-            const int quads = n >> 2, rest = n & 3;
-#pragma unroll 2
-            for (int i = 0; i < quads; i++) {
-                step(-1);
-                s += 4;
-            }
-            if (rest) {
-                s -= max(L.q - (rest - 1), 0);  // lanes past the end read element n - 1
-                step(L.q < rest ? -1 : 0);
-            }
-#pragma unroll
-            for (int j = 0; j < MT; j++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int l = (l0 + j) * 8 + L.r, ko = kf * 8 + 2 * L.q + e;
-                    if (l < nl && ko < nk) store(l, ko, re[j][e], im[j][e]);
-                }
-        });
-    }
-    rot = (rot + items) % kWarps;
-}
-
-// Half-spectrum to real (x axis, c2r) of a complex [line][k] plane, k < n/2+1: the chain of
-// output m starts at X(0).x and takes 2 X(k).x w.x, then -2 X(k).y w.y, for k = 1, 2, ...; at
-// the Nyquist frequency (2k = n) X(k).x w.x alone.
-template <typename F>
-__device__ __forceinline__ void c2r_plane(const double2* src, int sl, int n, int nl, const double2* tw, int& rot,
-                                          F&& store) {
-    const Lane L;
-    const int h = n / 2 + 1;
-    const int lf = (nl + 7) / 8, cf = (n + 7) / 8;
-    const int chunks = (lf + kRealChunk - 1) / kRealChunk, per = (lf + chunks - 1) / chunks;
-    const int items = cf * chunks;
-    for (int it = ((threadIdx.x >> 5) + kWarps - rot) % kWarps; it < items; it += kWarps) {
-        const int mf = it / chunks, l0 = (it - mf * chunks) * per;
-        __syncwarp();
-        dispatch<kRealChunk>(min(per, lf - l0), [&](auto mt) {
-            constexpr int MT = decltype(mt)::value;
-            double acc[MT][2];
-#pragma unroll
-            for (int j = 0; j < MT; j++) acc[j][0] = acc[j][1] = 0.0;
-            const int m = (mf * 8 + L.r) % n;
-            int t = L.dm ? m : 0;
-            const int inc = 2 * m >= n ? 2 * m - n : 2 * m;
-            const double* twd = reinterpret_cast<const double*>(tw);
-            const double* s = reinterpret_cast<const double*>(src + (l0 * 8 + L.r) * sl) + L.q;
-            const int pairs = (h + 1) >> 1;
-            for (int i = 0; i < pairs; i++) {
-                const int k = 2 * i + L.dm;
-                const int in = k < h ? -1 : 0;
-                const bool edge = k == 0 || 2 * k == n;
-                const double f = edge ? 1.0 : (L.p ? -2.0 : 2.0);
-                const int keep = edge && L.p ? 0 : in;
-                const double b = keep_or(twd[2 * t + L.p], in, 0);
-                t += inc;
-                if (t >= n) t -= n;
-                const double* e = s + (in ? 0 : -2);  // past the end: element h - 1
-#pragma unroll
-                for (int j = 0; j < MT; j++) mma_f64(acc[j], keep_or(f * e[16 * j * sl], keep, 1), b);
-                s += 4;
-            }
-#pragma unroll
-            for (int j = 0; j < MT; j++) {
-                const int l = (l0 + j) * 8 + L.r, mo = mf * 8 + 2 * L.q;
-                if (l < nl && mo < n) store(l, mo, acc[j][0]);
-                if (l < nl && mo + 1 < n) store(l, mo + 1, acc[j][1]);
-            }
-        });
-    }
-    rot = (rot + items) % kWarps;
-}
-
-// Which plane of a tile a flat line belongs to, n lines a plane.
-__device__ __forceinline__ int plane_of(int l, int n) {
-    int u = 0;
-#pragma unroll
-    for (int i = 1; i < kPlanes; i++) u += l >= i * n;
-    return u;
-}
-
-__device__ __forceinline__ void load_twiddles(double2* tw_s, const double2* __restrict__ tw, int n, int id, int step) {
-    for (int j = id; j < n; j += step) tw_s[j] = tw[j];
-}
-
-// Elements of u planes' buffers (the last fragment of lines may read up to 7 lines past the
-// end): [line][m] real, [m][line] complex, [line][k] complex.
-__host__ __device__ constexpr int real_planes(int n, int u) { return (u * n + 7) / 8 * 8 * pitch4(n) + 8; }
-__host__ __device__ constexpr int spec_planes_ml(int n, int u) { return n * pitch4(u * (n / 2 + 1)) + 8; }
-__host__ __device__ constexpr int spec_planes_lm(int n, int u) { return (u * n + 7) / 8 * 8 * pitch2(n / 2 + 1) + 4; }
-__host__ __device__ constexpr int pass_a_bytes(int n, int u) {
-    return 16 * (n + spec_planes_ml(n, u)) + 8 * real_planes(n, u);
-}
-__host__ __device__ constexpr int pass_c_bytes(int n, int u) {
-    const int pk = 16 * spec_planes_ml(n, u), xo = 8 * u * n * pitch4(n);
-    return 16 * (n + spec_planes_lm(n, u)) + (pk > xo ? pk : xo);
-}
-// Planes a tile takes together: as many as keep three CTAs on an SM.  The h = n/2 + 1 lines of
-// one plane fill their fragments badly (18 of 24 at n = 35); those of two or more planes run
-// on (36 of 40), and each block barrier covers more work.
-__host__ __device__ constexpr int tile_planes(int n) {
-    int u = 1;
-    while (u < kPlanes && pass_a_bytes(n, u + 1) <= kTileBytes && pass_c_bytes(n, u + 1) <= kTileBytes) u++;
-    return u;
-}
-
-// Pass A: x r2c then y forward, up to tile_planes(n) consecutive z-planes of a grain at a time.
-__global__ void __launch_bounds__(kThreads, 3) conv_pass_a(ConvArgs a) {
+__device__ __forceinline__ void warp_fragments(const ConvArgs& a, int warp_bytes, int per, bool rows, F&& f) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    int rot = 0;
-    for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid();) {
-        const int g = w.g, z = w.local;
-        const Box b = load_box(a.in_box + 6 * g);
-        const int n = b.nx(), h = n / 2 + 1;
-        const int U = min(min(tile_planes(n), w.count - z), w.end - w.t);
-        const int P = pitch4(n), Hp = pitch4(U * h);
-        double2* tw_s = reinterpret_cast<double2*>(smem_raw);
-        double2* A = tw_s + n;  // [y][plane, kx]
-        double* xp = reinterpret_cast<double*>(A + spec_planes_ml(n, U));  // [plane, y][x]
-        load_twiddles(tw_s, a.tw + a.tw_off[n], n, threadIdx.x, kThreads);
-        const double* src = a.in + a.in_off[g] + (long long)z * n * n;
-        for (int q = threadIdx.x; q < U * n * n; q += kThreads) {
-            const int y = q / n, x = q - y * n;
-            cp_async_elem(xp + y * P + x, src + q);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    double2* tw_s = reinterpret_cast<double2*>(smem_raw + (size_t)warp * warp_bytes);
+    const int parts = gridDim.x * warps, part = blockIdx.x * warps + warp;
+    const int share = a.toff[a.G + 1] < 2 * parts ? 4 : 1, mine = part % share;
+    if (part / share >= parts / share) return;
+    int n_tw = 0;
+    for (TileWalk w(a.toff, a.G, part / share, parts / share); w.valid(); w.next()) {
+        const int n = load_box(a.in_box + 6 * w.g).nx();
+        const int lines = rows ? n * n : n * (n / 2 + 1), frags = (lines + per - 1) / per;
+        if (n != n_tw) load_twiddles(tw_s, a.tw + a.tw_off[n], n, lane);
+        n_tw = n;
+        const long long t = (long long)w.local * share + mine, tiles = (long long)n * share;
+        const int f1 = (int)((t + 1) * frags / tiles);
+        for (int i = (int)(t * frags / tiles); i < f1; i++) f(w.g, n, tw_s, tw_s + n, i * per, lines);
+    }
+}
+
+// x forward: kRowFrags x 8 consecutive rows (z, y), each a chain per frequency k < n/2 + 1:
+// re = sum of x w.x, im = sum of x (-w.y).
+__global__ void __launch_bounds__(kThreads, 2) conv_x_forward(ConvArgs a, int warp_bytes) {
+    const Lane L;
+    warp_fragments(a, warp_bytes, 8 * kRowFrags, true, [&](int g, int n, const double2* tw, double2* buf, int r0, int rows) {
+        const int h = n / 2 + 1, P = pitch4(n), cf = (h + 7) / 8;
+        double* X = reinterpret_cast<double*>(buf);  // [row][x]
+        const double* src = a.in + a.in_off[g] + (long long)r0 * n;
+        const int count = min(8 * kRowFrags, rows - r0) * n;
+        for (int q = L.lane; q < count; q += 32) {
+            const int r = q / n;
+            cp_async_elem(X + r * P + (q - r * n), src + q);
         }
         cp_async_wait_all();
-        __syncthreads();
-        r2c_plane(xp, P, n, U * n, h, tw_s, rot, [&](int l, int k, double re, double im) {
-            const int u = plane_of(l, n);
-            A[(l - u * n) * Hp + u * h + k] = make_double2(re, im);
-        });
-        __syncthreads();
-        double2* dst = a.spec + a.spec_off[g] + (long long)z * n * h;
-        cdft_plane<false>(A, Hp, n, U * h, tw_s, rot, [&](int l, int ky, double re, double im) {
-            const int u = plane_of(l, h);
-            dst[(u * n + ky) * h + (l - u * h)] = make_double2(re, im);
-        });
-        __syncthreads();
-        for (int u = 0; u < U; u++) w.next();
-    }
-}
-
-// Pass B: z forward, Gaussian multiply, z inverse, 8 consecutive (ky, kx) lines per warp at a
-// time: a warp's lines, twiddles and products are its own, so nothing waits on a block
-// barrier.  A grain's n tiles share its n h lines in fragments of 8 without padding.
-__global__ void __launch_bounds__(kThreadsB, 2) conv_pass_b(ConvArgs a, int warp_bytes) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const Lane L;
-    const int warp = threadIdx.x >> 5;
-    double2* tw_s = reinterpret_cast<double2*>(smem_raw + (size_t)warp * warp_bytes);
-    const double* twd = reinterpret_cast<const double*>(tw_s);
-    int n_tw = 0;
-    const int warps = blockDim.x >> 5;
-    for (TileWalk w(a.toff, a.G, blockIdx.x * warps + warp, gridDim.x * warps); w.valid(); w.next()) {
-        const int g = w.g;
-        const Box b = load_box(a.in_box + 6 * g);
-        const int n = b.nx(), h = n / 2 + 1;
-        const int lines = n * h, frags = (lines + 7) / 8, cf = (n + 7) / 8;
-        if (n != n_tw) load_twiddles(tw_s, a.tw + a.tw_off[n], n, L.lane, 32);
-        n_tw = n;
-        double2* S = tw_s + n;
-        double2* T = cf > kColChunk ? S + n * kLP : S;  // one chunk: the products replace the lines in place
-        double2* spec = a.spec + a.spec_off[g];
-        const double* G = a.gtab + a.g_off[n];
-        const int f1 = (int)((long long)(w.local + 1) * frags / n);
-        for (int f = (int)((long long)w.local * frags / n); f < f1; f++) {
-            const int l0 = f * 8;
-            {
-                const int l = L.lane & 7;
-                if (l0 + l < lines)
-                    for (int z = L.lane >> 3; z < n; z += 4)
-                        cp_async16(S + z * kLP + l, spec + (long long)z * lines + l0 + l);
-            }
-            cp_async_wait_all();
+        __syncwarp();
+        double2* dst = a.spec + a.spec_off[g] + (long long)r0 * h;
+        for (int c0 = 0; c0 < cf; c0 += kRowChunk) {
             __syncwarp();
-            // this lane's products belong to line l0 + r
-            const int line = min(l0 + L.r, lines - 1), ky = line / h, kx = line - ky * h;
-            const int i2 = min(ky, n - ky), j2 = min(kx, n - kx), ij = i2 * i2 + j2 * j2;
-            for (int c0 = 0; c0 < cf; c0 += kColChunk)
-                dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
-                    constexpr int NT = decltype(nt)::value;
-                    double re[1][NT][2], im[1][NT][2];
-                    cdft<false, 1, NT>(reinterpret_cast<const double*>(S), 2 * kLP, n, c0, twd, L, re, im);
-                    __syncwarp();
+            dispatch<kRowChunk>(min(kRowChunk, cf - c0), [&](auto nt) {
+                constexpr int NT = decltype(nt)::value;
+                double re[kRowFrags][NT][2], im[kRowFrags][NT][2];
+                int t[NT], inc[NT];
+#pragma unroll
+                for (int c = 0; c < NT; c++) {
+                    const int k = ((c0 + c) * 8 + L.r) % n;
+                    t[c] = (L.q * k) % n;
+                    inc[c] = (4 * k) % n;
+#pragma unroll
+                    for (int j = 0; j < kRowFrags; j++) re[j][c][0] = re[j][c][1] = im[j][c][0] = im[j][c][1] = 0.0;
+                }
+                const double* s = X + L.r * P + L.q;
+                auto step = [&](int keep) {
+                    double x[kRowFrags];
+#pragma unroll
+                    for (int j = 0; j < kRowFrags; j++) x[j] = keep_or(s[8 * j * P], keep, 1);
+#pragma unroll
+                    for (int c = 0; c < NT; c++) {
+                        const double2 w = tw[t[c]];
+                        const double wx = keep_or(w.x, keep, 0), wy = keep_or(-w.y, keep, 0);
+                        t[c] += inc[c];
+                        if (t[c] >= n) t[c] -= n;
+#pragma unroll
+                        for (int j = 0; j < kRowFrags; j++) {
+                            mma_f64(re[j][c], x[j], wx);
+                            mma_f64(im[j][c], x[j], wy);
+                        }
+                    }
+                };
+                const int quads = n >> 2, rest = n & 3;
+#pragma unroll 2
+                for (int i = 0; i < quads; i++) {
+                    step(-1);
+                    s += 4;
+                }
+                if (rest) {
+                    s -= max(L.q - (rest - 1), 0);  // lanes past the end read element n - 1
+                    step(L.q < rest ? -1 : 0);
+                }
+#pragma unroll
+                for (int j = 0; j < kRowFrags; j++)
 #pragma unroll
                     for (int c = 0; c < NT; c++)
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
-                            const int kz = (c0 + c) * 8 + 2 * L.q + e;
-                            if (kz < n) {
-                                const int k2 = min(kz, n - kz);
-                                const double gv = __ldg(G + (ij + k2 * k2));
-                                T[kz * kLP + L.r] = make_double2(re[0][c][e] * gv, im[0][c][e] * gv);
-                            }
+                            const int r = 8 * j + L.r, k = (c0 + c) * 8 + 2 * L.q + e;
+                            if (r0 + r < rows && k < h) dst[r * h + k] = make_double2(re[j][c][e], im[j][c][e]);
                         }
-                });
-            __syncwarp();
-            for (int c0 = 0; c0 < cf; c0 += kColChunk)
-                dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
-                    constexpr int NT = decltype(nt)::value;
-                    double re[1][NT][2], im[1][NT][2];
-                    cdft<true, 1, NT>(reinterpret_cast<const double*>(T), 2 * kLP, n, c0, twd, L, re, im);
-                    if (l0 + L.r < lines) {
-#pragma unroll
-                        for (int c = 0; c < NT; c++)
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const int z = (c0 + c) * 8 + 2 * L.q + e;
-                                if (z < n)
-                                    spec[(long long)z * lines + l0 + L.r] = make_double2(re[0][c][e], im[0][c][e]);
-                            }
-                    }
-                });
-            __syncwarp();
+            });
         }
-    }
+        __syncwarp();
+    });
 }
 
-// Pass C: y inverse then x c2r, the planes of a tile as in pass A, written to the output arena.
-__global__ void __launch_bounds__(kThreads, 3) conv_pass_c(ConvArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    int rot = 0;
-    for (TileWalk w(a.toff, a.G, blockIdx.x, gridDim.x); w.valid();) {
-        const int g = w.g, z = w.local;
-        const Box b = load_box(a.in_box + 6 * g);
-        const int n = b.nx(), h = n / 2 + 1;
-        const int U = min(min(tile_planes(n), w.count - z), w.end - w.t);
-        const int P = pitch4(n), Hp = pitch4(U * h), Hl = pitch2(h);
-        double2* tw_s = reinterpret_cast<double2*>(smem_raw);
-        double2* Ay = tw_s + n;                      // [plane, y][kx], pitch Hl
-        double2* Pk = Ay + spec_planes_lm(n, U);     // [ky][plane, kx], pitch Hp
-        double* xo = reinterpret_cast<double*>(Pk);  // [plane, y][x], pitch P, once the spectrum is read
-        load_twiddles(tw_s, a.tw + a.tw_off[n], n, threadIdx.x, kThreads);
-        const double2* spec = a.spec + a.spec_off[g] + (long long)z * n * h;
-        for (int q = threadIdx.x; q < U * n * h; q += kThreads) {
-            const int row = q / h, kx = q - row * h, u = plane_of(row, n);
-            cp_async16(Pk + (row - u * n) * Hp + u * h + kx, spec + q);
+// Stages 8 lines (the one of lane l & 7 at src, elements `stride` apart) as [m][line].
+__device__ __forceinline__ void stage_lines(double2* S, const double2* src, bool have, int n, int stride, int lane) {
+    if (have)
+        for (int m = lane >> 3; m < n; m += 4) cp_async16(S + m * kLP + (lane & 7), src + (long long)m * stride);
+    cp_async_wait_all();
+    __syncwarp();
+}
+
+// y, forward or inverse, in place: 8 consecutive lines (z, kx).
+template <bool INV>
+__global__ void __launch_bounds__(kThreads, 2) conv_y(ConvArgs a, int warp_bytes) {
+    const Lane L;
+    warp_fragments(a, warp_bytes, 8, false, [&](int g, int n, const double2* tw, double2* S, int l0, int lines) {
+        const int h = n / 2 + 1, cf = (n + 7) / 8;
+        double2* spec = a.spec + a.spec_off[g];
+        auto line_at = [&](int l) {  // line (z, kx) starts at z n h + kx
+            const int z = l / h;
+            return spec + (z * n * h + (l - z * h));
+        };
+        stage_lines(S, line_at(min(l0 + (L.lane & 7), lines - 1)), l0 + (L.lane & 7) < lines, n, h, L.lane);
+        double2* dst = line_at(min(l0 + L.r, lines - 1));
+        for (int c0 = 0; c0 < cf; c0 += kColChunk) {
+            __syncwarp();
+            dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
+                constexpr int NT = decltype(nt)::value;
+                double re[1][NT][2], im[1][NT][2];
+                cdft<INV, 1, NT>(reinterpret_cast<const double*>(S), 2 * kLP, n, c0, reinterpret_cast<const double*>(tw), L,
+                                 re, im);
+                if (l0 + L.r < lines) {
+#pragma unroll
+                    for (int c = 0; c < NT; c++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int k = (c0 + c) * 8 + 2 * L.q + e;
+                            if (k < n) dst[k * h] = make_double2(re[0][c][e], im[0][c][e]);
+                        }
+                }
+            });
+        }
+        __syncwarp();
+    });
+}
+
+// z forward, Gaussian multiply, z inverse, in place: 8 consecutive lines (ky, kx).
+__global__ void __launch_bounds__(kThreads, 2) conv_z(ConvArgs a, int warp_bytes) {
+    const Lane L;
+    warp_fragments(a, warp_bytes, 8, false, [&](int g, int n, const double2* tw, double2* S, int l0, int lines) {
+        const int h = n / 2 + 1, cf = (n + 7) / 8;
+        const double* twd = reinterpret_cast<const double*>(tw);
+        double2* T = cf > kColChunk ? S + n * kLP : S;  // one chunk: the products replace the lines in place
+        double2* spec = a.spec + a.spec_off[g];
+        const double* G = a.gtab + a.g_off[n];
+        stage_lines(S, spec + min(l0 + (L.lane & 7), lines - 1), l0 + (L.lane & 7) < lines, n, lines, L.lane);
+        // this lane's products belong to line l0 + r
+        const int line = min(l0 + L.r, lines - 1), ky = line / h, kx = line - ky * h;
+        const int i2 = min(ky, n - ky), j2 = min(kx, n - kx), ij = i2 * i2 + j2 * j2;
+        for (int c0 = 0; c0 < cf; c0 += kColChunk) {
+            __syncwarp();
+            dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
+                constexpr int NT = decltype(nt)::value;
+                double re[1][NT][2], im[1][NT][2];
+                cdft<false, 1, NT>(reinterpret_cast<const double*>(S), 2 * kLP, n, c0, twd, L, re, im);
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < NT; c++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const int kz = (c0 + c) * 8 + 2 * L.q + e;
+                        if (kz < n) {
+                            const int k2 = min(kz, n - kz);
+                            const double gv = __ldg(G + (ij + k2 * k2));
+                            T[kz * kLP + L.r] = make_double2(re[0][c][e] * gv, im[0][c][e] * gv);
+                        }
+                    }
+            });
+        }
+        __syncwarp();
+        for (int c0 = 0; c0 < cf; c0 += kColChunk) {
+            __syncwarp();
+            dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
+                constexpr int NT = decltype(nt)::value;
+                double re[1][NT][2], im[1][NT][2];
+                cdft<true, 1, NT>(reinterpret_cast<const double*>(T), 2 * kLP, n, c0, twd, L, re, im);
+                if (l0 + L.r < lines) {
+#pragma unroll
+                    for (int c = 0; c < NT; c++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int z = (c0 + c) * 8 + 2 * L.q + e;
+                            if (z < n) spec[(long long)z * lines + l0 + L.r] = make_double2(re[0][c][e], im[0][c][e]);
+                        }
+                }
+            });
+        }
+        __syncwarp();
+    });
+}
+
+// x inverse (half spectrum to real): the chain of output m starts at X(0).x and takes 2 X(k).x
+// w.x, then -2 X(k).y w.y, for k = 1, 2, ...; at the Nyquist frequency (2k = n) X(k).x w.x alone.
+__global__ void __launch_bounds__(kThreads, 2) conv_x_inverse(ConvArgs a, int warp_bytes) {
+    const Lane L;
+    warp_fragments(a, warp_bytes, 8 * kRowFrags, true, [&](int g, int n, const double2* tw, double2* X, int r0, int rows) {
+        const int h = n / 2 + 1, P = pitch2(h), cf = (n + 7) / 8;
+        const double* twd = reinterpret_cast<const double*>(tw);
+        const double2* src = a.spec + a.spec_off[g] + (long long)r0 * h;  // X: [row][k]
+        const int count = min(8 * kRowFrags, rows - r0) * h;
+        for (int q = L.lane; q < count; q += 32) {
+            const int r = q / h;
+            cp_async16(X + r * P + (q - r * h), src + q);
         }
         cp_async_wait_all();
-        __syncthreads();
-        cdft_plane<true>(Pk, Hp, n, U * h, tw_s, rot, [&](int l, int y, double re, double im) {
-            const int u = plane_of(l, h);
-            Ay[(u * n + y) * Hl + (l - u * h)] = make_double2(re, im);
-        });
-        __syncthreads();
-        c2r_plane(Ay, Hl, n, U * n, tw_s, rot, [&](int l, int x, double v) { xo[l * P + x] = v; });
-        __syncthreads();
-        double* dst = a.out + a.out_off[g] + (long long)z * n * n;
-        for (int q = threadIdx.x; q < U * n * n; q += kThreads) {
-            const int y = q / n, x = q - y * n;
-            dst[q] = xo[y * P + x];
+        __syncwarp();
+        double* dst = a.out + a.out_off[g] + (long long)r0 * n;
+        for (int c0 = 0; c0 < cf; c0 += kColChunk) {
+            __syncwarp();
+            dispatch<kColChunk>(min(kColChunk, cf - c0), [&](auto nt) {
+                constexpr int NT = decltype(nt)::value;
+                double acc[kRowFrags][NT][2];
+                int t[NT], inc[NT];
+#pragma unroll
+                for (int c = 0; c < NT; c++) {
+                    const int m = ((c0 + c) * 8 + L.r) % n;
+                    t[c] = L.dm ? m : 0;
+                    inc[c] = 2 * m >= n ? 2 * m - n : 2 * m;
+#pragma unroll
+                    for (int j = 0; j < kRowFrags; j++) acc[j][c][0] = acc[j][c][1] = 0.0;
+                }
+                const double* s = reinterpret_cast<const double*>(X + L.r * P) + L.q;
+                const int pairs = (h + 1) >> 1;
+#pragma unroll 2
+                for (int i = 0; i < pairs; i++) {
+                    const int k = 2 * i + L.dm;
+                    const int in = k < h ? -1 : 0;
+                    const bool edge = k == 0 || 2 * k == n;
+                    const double f = edge ? 1.0 : (L.p ? -2.0 : 2.0);
+                    const int keep = edge && L.p ? 0 : in;
+                    const double* e = s + (in ? 0 : -2);  // past the end: element h - 1
+                    double x[kRowFrags];
+#pragma unroll
+                    for (int j = 0; j < kRowFrags; j++) x[j] = keep_or(f * e[16 * j * P], keep, 1);
+#pragma unroll
+                    for (int c = 0; c < NT; c++) {
+                        const double b = keep_or(twd[2 * t[c] + L.p], in, 0);
+                        t[c] += inc[c];
+                        if (t[c] >= n) t[c] -= n;
+#pragma unroll
+                        for (int j = 0; j < kRowFrags; j++) mma_f64(acc[j][c], x[j], b);
+                    }
+                    s += 4;
+                }
+#pragma unroll
+                for (int j = 0; j < kRowFrags; j++)
+#pragma unroll
+                    for (int c = 0; c < NT; c++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int r = 8 * j + L.r, m = (c0 + c) * 8 + 2 * L.q + e;
+                            if (r0 + r < rows && m < n) dst[r * n + m] = acc[j][c][e];
+                        }
+            });
         }
-        __syncthreads();
-        for (int u = 0; u < U; u++) w.next();
-    }
+        __syncwarp();
+    });
 }
 
-constexpr size_t kMaxSmem = 227 * 1024;
-size_t pass_b_warp_bytes(int n) {
-    return 16 * (size_t)n * (1 + kLP * ((n + 7) / 8 > kColChunk ? 2 : 1)) + 16 * 8;
-}
+// Shared memory of a warp of each pass, in bytes, at side n: its twiddles and its lines (and
+// z's products, above kColChunk fragments).
+constexpr int kSlack = 16 * 8;
+int x_forward_bytes(int n) { return 16 * n + 8 * 8 * kRowFrags * pitch4(n) + kSlack; }
+int y_bytes(int n) { return 16 * n * (1 + kLP) + kSlack; }
+int z_bytes(int n) { return 16 * n * (1 + kLP * ((n + 7) / 8 > kColChunk ? 2 : 1)) + kSlack; }
+int x_inverse_bytes(int n) { return 16 * n + 16 * 8 * kRowFrags * pitch2(n / 2 + 1) + kSlack; }
 
-// CTAs of kernel k: a whole number of waves of those that fit the device at once, near
-// `grid` (a wave that is two thirds empty at the end cost 11% of a pass).
+// CTAs of as many warps as fit (8 at most), whole waves of the CTAs that fit the device at once:
+// one wave for a few boxes, where every wave pays its start (0.100 -> 0.082 ms for 20 grains of
+// 32^3 against four), up to eight, which even out the boxes' sides, for many (3.95 -> 3.52 ms
+// for 2,000 of 128^3 against one).
 template <typename K>
-int whole_waves(K kernel, int threads, size_t smem, int grid) {
+void launch_pass(K kernel, const ConvArgs& a, int warp_bytes, int nmax, cudaStream_t s) {
+    constexpr int kMaxSmem = 227 * 1024;
+    const int warps = std::min(kMaxSmem / warp_bytes, kWarps);
+    const size_t smem = (size_t)warps * warp_bytes;
     int dev = 0, sms = 148, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * warps, smem);
     const int wave = sms * (per_sm > 0 ? per_sm : 1);
-    return wave * (grid > wave ? (grid + wave / 2) / wave : 1);
+    const long long tiles = (long long)a.G * nmax;  // at most
+    const int waves = (int)std::min(8LL, std::max(1LL, tiles / (4LL * wave * warps)));
+    kernel<<<wave * waves, 32 * warps, smem, s>>>(a, warp_bytes);
 }
 
 }  // namespace
 
-void launch_conv_f64(const ConvArgs& a, int grid, int nmax, cudaStream_t s) {
+void launch_conv_f64(const ConvArgs& a, int nmax, cudaStream_t s) {
     static PerDevice configured;
     configured.once([] {
-        allow_max_dynamic_smem(conv_pass_a);
-        allow_max_dynamic_smem(conv_pass_b);
-        allow_max_dynamic_smem(conv_pass_c);
+        allow_max_dynamic_smem(conv_x_forward);
+        allow_max_dynamic_smem(conv_y<false>);
+        allow_max_dynamic_smem(conv_z);
+        allow_max_dynamic_smem(conv_y<true>);
+        allow_max_dynamic_smem(conv_x_inverse);
     });
-    // a tile of several planes of a smaller side may need more than one plane of the largest
-    size_t sa = 0, sc = 0;
-    for (int n = 1; n <= nmax; n++) {
-        sa = std::max(sa, (size_t)pass_a_bytes(n, tile_planes(n)));
-        sc = std::max(sc, (size_t)pass_c_bytes(n, tile_planes(n)));
-    }
-    const int warp_bytes = (int)pass_b_warp_bytes(nmax);
-    // sides above 64 keep two line buffers a warp, and as many warps as then fit
-    const int warps = std::min((int)(kMaxSmem / warp_bytes), kThreadsB / 32);
-    const size_t sb = (size_t)warps * warp_bytes;
-    conv_pass_a<<<whole_waves(conv_pass_a, kThreads, sa, grid), kThreads, sa, s>>>(a);
-    conv_pass_b<<<whole_waves(conv_pass_b, 32 * warps, sb, grid), 32 * warps, sb, s>>>(a, warp_bytes);
-    conv_pass_c<<<whole_waves(conv_pass_c, kThreads, sc, grid), kThreads, sc, s>>>(a);
+    launch_pass(conv_x_forward, a, x_forward_bytes(nmax), nmax, s);
+    launch_pass(conv_y<false>, a, y_bytes(nmax), nmax, s);
+    launch_pass(conv_z, a, z_bytes(nmax), nmax, s);
+    launch_pass(conv_y<true>, a, y_bytes(nmax), nmax, s);
+    launch_pass(conv_x_inverse, a, x_inverse_bytes(nmax), nmax, s);
 }
 
 }  // namespace gg

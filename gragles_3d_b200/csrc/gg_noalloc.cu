@@ -154,9 +154,8 @@ extern "C" int gg_convolve_boxes_f64_noalloc(const double* d_in, double* d_out, 
         spec_total += (long long)n * n * (n / 2 + 1);
     }
     if (spec_total > kScratchComplex) return GG_ERR_UNSUPPORTED;
-    int dev = 0, sms = 0;
+    int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return GG_ERR_CUDA;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceState& d = g_dev[dev];
@@ -200,7 +199,7 @@ extern "C" int gg_convolve_boxes_f64_noalloc(const double* d_in, double* d_out, 
     // an error left over from earlier, unrelated work is not this launch's: clear it
     // first (a sticky error has already failed the copies above)
     (void)cudaGetLastError();
-    gg::launch_conv_f64(a, (sms > 0 ? sms : 148) * 8, nmax, 0);
+    gg::launch_conv_f64(a, nmax, 0);
     if (cudaGetLastError() != cudaSuccess) return GG_ERR_CUDA;
     if (cudaDeviceSynchronize() != cudaSuccess) return GG_ERR_CUDA;
     return GG_OK;
