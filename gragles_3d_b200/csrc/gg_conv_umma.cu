@@ -163,6 +163,20 @@ struct Cursor {
     __device__ int rows() const { return min(kRows, n * n - local * kRows); }
 };
 
+// Position in a ring of `size` slots and the phase parity of its barriers, advanced tile by
+// tile: i % size and (i / size) & 1 without the divisions, which each role would have on the
+// critical path of every tile.
+struct Ring {
+    int size, slot, phase;
+    __device__ explicit Ring(int n) : size(n), slot(0), phase(0) {}
+    __device__ void next() {
+        if (++slot == size) {
+            slot = 0;
+            phase ^= 1;
+        }
+    }
+};
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
 }
@@ -211,28 +225,51 @@ __device__ __forceinline__ void drain_bar(uint32_t bar, uint32_t parity, int* er
 // a thread writes one such row (lane % 8 = row, lane / 8 picks one of four
 // consecutive core matrices), so each 8-lane phase stores one whole core matrix.
 // Padding rows and columns become zero.
-__device__ __forceinline__ void split_tile(const float* raw, __half* hi, __half* lo, int n, int rows, int stid) {
-    const int KC = round_k(n) >> 3;
-    const int w = stid >> 5, lane = stid & 31;
-    const int r = lane & 7, j = lane >> 3;
+// A thread's core matrices, first q and stride 4 kSplitWarps, as (mg, kc) steps: worked out when
+// the side changes, not by a division per core matrix.
+struct SplitPlan {
+    int n, KC, mg0, kc0, dmg, dkc;
+    __device__ void set(int side, int stid) {
+        n = side;
+        KC = round_k(n) >> 3;
+        const int q0 = 4 * (stid >> 5) + ((stid & 31) >> 3);
+        mg0 = q0 / KC;
+        kc0 = q0 - mg0 * KC;
+        dmg = 4 * kSplitWarps / KC;
+        dkc = 4 * kSplitWarps - dmg * KC;
+    }
+};
+__device__ __forceinline__ void split_tile(const float* raw, __half* hi, __half* lo, const SplitPlan& P, int rows,
+                                           int stid) {
+    const int r = stid & 7, n = P.n;
     const bool vec = (n & 3) == 0;  // rows start on 16-byte boundaries
-    for (int q = 4 * w + j; q < 16 * KC; q += 4 * kSplitWarps) {
-        const int mg = q / KC, kc = q - mg * KC;
+    int mg = P.mg0, kc = P.kc0;
+    for (; mg < kRows / 8; mg += P.dmg, kc += P.dkc) {
+        if (kc >= P.KC) {
+            kc -= P.KC;
+            if (++mg >= kRows / 8) break;
+        }
         const int m = 8 * mg + r, k0 = 8 * kc;
+        const float* src = raw + m * n + k0;
         float v[8];
-        if (m < rows && vec && k0 + 8 <= n) {
-            const float4 a = *reinterpret_cast<const float4*>(raw + m * n + k0);
-            const float4 b = *reinterpret_cast<const float4*>(raw + m * n + k0 + 4);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        if (m < rows && k0 + 8 <= n) {
+            if (vec) {
+                const float4 a = *reinterpret_cast<const float4*>(src);
+                const float4 b = *reinterpret_cast<const float4*>(src + 4);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = src[e];
+            }
         } else {
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = (m < rows && k0 + e < n) ? raw[m * n + k0 + e] : 0.f;
+            for (int e = 0; e < 8; e++) v[e] = (m < rows && k0 + e < n) ? src[e] : 0.f;
         }
         __align__(16) __half2 hv[4], lv[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) split_f16x2(v[2 * e], v[2 * e + 1], hv[e], lv[e]);
-        const int off = q * 64 + r * 8;  // halves
+        const int off = (mg * P.KC + kc) * 64 + r * 8;  // halves
         *reinterpret_cast<uint4*>(hi + off) = *reinterpret_cast<const uint4*>(hv);
         *reinterpret_cast<uint4*>(lo + off) = *reinterpret_cast<const uint4*>(lv);
     }
@@ -306,12 +343,16 @@ __global__ void __launch_bounds__(kThreadsU, 1)
         // ---------------- split ----------------
         Cursor c;
         c.init(&a, t_begin);
-        for (int i = 0; i < count; i++, c.advance()) {
-            const int r = i % R, s = i % S;
-            if (!wait_bar(bar(RFULL + r), (i / R) & 1, ab, a.err)) break;
-            if (i >= S && !wait_bar(bar(EMPTY + s), (i / S - 1) & 1, ab, a.err)) break;
+        SplitPlan plan;
+        plan.n = 0;
+        Ring rr(R), rs(S);
+        for (int i = 0; i < count; i++, c.advance(), rr.next(), rs.next()) {
+            const int r = rr.slot, s = rs.slot;
+            if (c.n != plan.n) plan.set(c.n, tid);
+            if (!wait_bar(bar(RFULL + r), rr.phase, ab, a.err)) break;
+            if (i >= S && !wait_bar(bar(EMPTY + s), rs.phase ^ 1, ab, a.err)) break;
             __half* hi = op_base + s * 2 * tile_halves;
-            split_tile(raw_base + r * tile_floats, hi, hi + tile_halves, c.n, c.rows(), tid);
+            split_tile(raw_base + r * tile_floats, hi, hi + tile_halves, plan, c.rows(), tid);
             // every lane's stores visible to the tensor core, then one arrive per warp
             // (arrives on one barrier serialise, so 256 of them would cost microseconds)
             fence_proxy_async();
@@ -328,9 +369,10 @@ __global__ void __launch_bounds__(kThreadsU, 1)
         Cursor c;
         c.init(&a, t_begin);
         if (e) c.advance();
+        static_assert((kAcc & (kAcc - 1)) == 0, "ring positions by masks");
         for (int i = e; i < count; i += 2, c.advance(), c.advance()) {
-            const int b = i % kAcc;
-            if (!wait_bar(bar(TFULL + b), (i / kAcc) & 1, ab, a.err)) break;
+            const int b = i & (kAcc - 1);
+            if (!wait_bar(bar(TFULL + b), ((unsigned)i / kAcc) & 1, ab, a.err)) break;
             tc_fence_after();
             const int n = c.n, np = round_n(n);
             const int row = q * 32 + lane;
@@ -359,33 +401,44 @@ __global__ void __launch_bounds__(kThreadsU, 1)
         // ---------------- MMA issue ----------------
         Cursor c;
         c.init(&a, t_begin);
-        int cur_n = -1, nsw = 0, kb = 0;
+        int cur_n = -1, nsw = 0, kb = 0, steps = 0;
         bool issued = false;
-        for (int i = 0; i < count; i++, c.advance()) {
-            const int s = i % S, b = i % kAcc;
-            if (!wait_bar(bar(FULL + s), (i / S) & 1, ab, a.err)) break;
+        uint32_t idesc = 0;
+        uint64_t b_hi = 0, b_lo = 0, fixed = 0;  // descriptors: C_n, and all but the address of the operands'
+        Ring rs(S), rb(kAcc);
+        for (int i = 0; i < count; i++, c.advance(), rs.next(), rb.next()) {
+            const int s = rs.slot, b = rb.slot;
+            if (!wait_bar(bar(FULL + s), rs.phase, ab, a.err)) break;
             if (c.n != cur_n) {
                 kb = nsw & 1;
                 if (nsw >= 1) mma_commit(bar(BFREE + (kb ^ 1)));  // after every MMA on the old C_n
                 if (!wait_bar(bar(BFULL + kb), (nsw >> 1) & 1, ab, a.err)) break;
                 cur_n = c.n;
                 nsw++;
+                const int kp = round_k(c.n), np = round_n(c.n);
+                const uint32_t sbo = 16u * kp;  // 8 rows x kp halves
+                const __half* bk = b_base + kb * b_halves;
+                fixed = smem_desc(0, sbo);
+                b_hi = smem_desc(smem_u32(bk), sbo);
+                b_lo = smem_desc(smem_u32(bk + np * kp), sbo);
+                idesc = instr_desc(np);
+                steps = kp / 16;
             }
-            if (i >= kAcc && !wait_bar(bar(TEMPTY + b), (i / kAcc - 1) & 1, ab, a.err)) break;
+            if (i >= kAcc && !wait_bar(bar(TEMPTY + b), rb.phase ^ 1, ab, a.err)) break;
             tc_fence_after();
-            const int kp = round_k(c.n), np = round_n(c.n);
-            const uint32_t sbo = 16u * kp;  // 8 rows x kp halves
-            const __half* hi = op_base + s * 2 * tile_halves;
-            const uint32_t a_hi = smem_u32(hi), a_lo = smem_u32(hi + tile_halves);
-            const __half* bk = b_base + kb * b_halves;
-            const uint32_t b_hi = smem_u32(bk), b_lo = smem_u32(bk + np * kp);
-            const uint32_t idesc = instr_desc(np);
+            const uint32_t op = smem_u32(op_base) + (uint32_t)(s * 2 * tile_halves) * 2u;
+            uint64_t a_hi = fixed | (op >> 4), a_lo = fixed | ((op + (uint32_t)tile_halves * 2u) >> 4);
+            uint64_t k_hi = b_hi, k_lo = b_lo;
             const uint32_t d = tmem + (uint32_t)(b * kAccCols);
-            for (int j = 0; j < kp / 16; j++) {
-                const uint32_t o = 256u * j;  // two 128-B core matrices along K
-                mma_f16(d, smem_desc(a_lo + o, sbo), smem_desc(b_hi + o, sbo), idesc, j > 0);
-                mma_f16(d, smem_desc(a_hi + o, sbo), smem_desc(b_lo + o, sbo), idesc, 1);
-                mma_f16(d, smem_desc(a_hi + o, sbo), smem_desc(b_hi + o, sbo), idesc, 1);
+            for (int j = 0; j < steps; j++) {
+                mma_f16(d, a_lo, k_hi, idesc, j > 0);
+                mma_f16(d, a_hi, k_lo, idesc, 1);
+                mma_f16(d, a_hi, k_hi, idesc, 1);
+                // two 128-B core matrices along K
+                a_hi += 16;
+                a_lo += 16;
+                k_hi += 16;
+                k_lo += 16;
             }
             issued = true;
             mma_commit(bar(EMPTY + s));
@@ -401,9 +454,10 @@ __global__ void __launch_bounds__(kThreadsU, 1)
         c.init(&a, t_begin);
         int cur_n = -1, nsw = 0;
         int last_tile[kMaxR] = {-1, -1, -1, -1}, last_b[2] = {-1, -1};  // last copy into each buffer
-        for (int i = 0; i < count; i++, c.advance()) {
-            const int r = i % R;
-            if (i >= R && !wait_bar(bar(REMPTY + r), (i / R - 1) & 1, ab, a.err)) break;
+        Ring rr(R);
+        for (int i = 0; i < count; i++, c.advance(), rr.next()) {
+            const int r = rr.slot;
+            if (i >= R && !wait_bar(bar(REMPTY + r), rr.phase ^ 1, ab, a.err)) break;
             if (c.n != cur_n) {
                 const int kb = nsw & 1;
                 if (nsw >= 2 && !wait_bar(bar(BFREE + kb), ((nsw - 2) >> 1) & 1, ab, a.err)) break;
