@@ -115,7 +115,7 @@ struct gg_ctx {
     int coarse_ref = 0, points_per_grain = 0;
     // launch configuration: CTAs per SM of each stage's grid-stride kernels (convolution
     // with the correction, lists, comparison, level set, redistancing), chosen by the
-    // autotuner when it is on
+    // autotuner when it is on; the comparison launches a fixed multiple of its entry
     int mult[5] = {8, 8, 4, 8, 8};
     int tune_next = -1;         // candidate the next tuning step runs, -1: not tuning
     double tune_cost[5][8] = {};

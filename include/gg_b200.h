@@ -122,7 +122,8 @@ int gg_step(gg_ctx* ctx, gg_step_stats* stats);
 int gg_domain_size(gg_ctx* ctx);
 
 /* The launch configuration in use: CTAs per SM of the grid-stride kernels of each stage
- * (convolution with the correction, lists, comparison, level set, redistancing).  No
+ * (convolution with the correction, lists, comparison, level set, redistancing; the
+ * comparison's grid is up to 16 times its entry, a CTA a share of the tiles).  No
  * counterpart in the reference (its parallel loops are OpenMP over grains).  Returns 1
  * once the autotuner has chosen them (or when it is off), 0 while it is still trying. */
 int gg_launch_config(gg_ctx* ctx, int32_t ctas_per_sm[5]);
