@@ -10,7 +10,8 @@
  *
  * Conventions: every function returns GG_OK (0) or a negative GG_ERR_* code and
  * never throws; gg_last_error() gives the message.  One context = one GPU, one
- * CUDA stream, one host thread.  Boxes are int32[6] = {xmin, xmax, ymin, ymax,
+ * CUDA stream (work that a step forks to streams of the context's own is joined to it before
+ * the call ends), one host thread.  Boxes are int32[6] = {xmin, xmax, ymin, ymax,
  * zmin, zmax} in absolute grid coordinates (border included), maxima exclusive,
  * and box buffers are flat [z][y][x] with x fastest (dimensionalBuffer.h:71-76).
  * Grain IDs run 1..n_grains; ID 0 is the domain-boundary grain.
@@ -71,6 +72,9 @@ typedef struct {
     int32_t live_grains;        /* grains whose hull is non-empty after the step */
     int32_t kernel_launches;    /* kernels this library launched for the step */
     int64_t voxel_updates;      /* sum of n^3 over the boxes convolved this step */
+    /* per-stage device times.  The interfacial-element build runs beside the redistancing
+     * when the grains are few for the GPU: ms_levelset then ends before it, and
+     * ms_redistancing includes what is left of it after the sweeps. */
     float ms_convolution, ms_lists, ms_comparison, ms_levelset, ms_redistancing, ms_total;
     float ms_compare_kernel;    /* the comparison kernel alone (device time) */
     int64_t compare_voxels;     /* box voxels that kernel compared */
