@@ -697,10 +697,10 @@ int level_set_t(gg_ctx* ctx, int p, int regrid) {
         e.err = ctx->d_err;
         // The redistancing does not need the elements, so the build, whose warps (six an SM, one
         // a grain) leave most of the device idle at its end or throughout, runs beside it on a
-        // stream of its own: level set and redistancing 7.7 -> 6.6 ms for 30 grains of 90^3 (4.7 since
-        // the build's loads run ahead), 3.15
-        // -> 2.97 for 1,900, 12.6 -> 12.4 for 8,400.  With more turns a warp both mostly take
-        // turns and disturb each other: 19.2 -> 19.9 ms for 20,000.
+        // stream of its own: level set and redistancing 7.7 -> 6.6 ms for 30 grains of 90^3 (4.7
+        // since the build's loads run ahead), 3.15 -> 2.97 for 1,900, 12.6 -> 12.4 for 8,400.
+        // With more turns a warp both mostly take turns and disturb each other: 19.2 -> 19.9 ms
+        // for 20,000.
         constexpr int kTurns = 12, kWarpsSM = 6;
         ctx->el_beside = ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
         cudaStream_t t = ctx->el_beside ? ctx->el_stream : ctx->stream;
