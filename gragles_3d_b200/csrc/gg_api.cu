@@ -252,10 +252,19 @@ int upload_tables(gg_ctx* ctx) {
     return rc;
 }
 
+int read_err(gg_ctx* ctx, int* e) {
+    CK(cudaMemcpyAsync(e, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return GG_OK;
+}
+
 int check_err(gg_ctx* ctx, const char* where) {
     int e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    if (const int rc = read_err(ctx, &e)) return rc;
+    if (e && ctx->el_beside) {  // a build beside the stream may still be adding its bits and naming its capacity
+        CK(cudaStreamSynchronize(ctx->el_stream));
+        if (const int rc = read_err(ctx, &e)) return rc;
+    }
     if (e & ERR_POOL) return fail(ctx, GG_ERR_POOL_EXHAUSTED, "%s: box pool or scratch capacity exceeded", where);
     if (e & (ERR_LIST | ERR_HASH)) return fail(ctx, GG_ERR_LIST_OVERFLOW, "%s: comparison list capacity exceeded", where);
     if (e & ERR_NEIGHBORS) return fail(ctx, GG_ERR_LIST_OVERFLOW, "%s: hull neighbour capacity exceeded", where);
@@ -702,16 +711,17 @@ int level_set_t(gg_ctx* ctx, int p, int regrid) {
         // With more turns a warp both mostly take turns and disturb each other: 19.2 -> 19.9 ms
         // for 20,000.
         constexpr int kTurns = 12, kWarpsSM = 6;
-        ctx->el_beside = ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
-        cudaStream_t t = ctx->el_beside ? ctx->el_stream : ctx->stream;
-        if (ctx->el_beside) {
+        const bool beside = ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
+        cudaStream_t t = beside ? ctx->el_stream : ctx->stream;
+        if (beside) {
             CK(cudaEventRecord(ctx->el_fork, ctx->stream));
             CK(cudaStreamWaitEvent(t, ctx->el_fork, 0));
         }
         launch_elements(e, ctx->elscr_ctas, t);
         ctx->launches += 1;
         CK(cudaGetLastError());
-        if (ctx->el_beside) CK(cudaEventRecord(ctx->el_join, t));
+        if (beside) CK(cudaEventRecord(ctx->el_join, t));
+        ctx->el_beside = beside;
     }
     return GG_OK;
 }
@@ -860,11 +870,15 @@ int step_t(gg_ctx* ctx, gg_step_stats* st) {
     if ((rc = stage_level_set_t<T>(ctx))) return rc;
     cudaEventRecord(ctx->ev[4], ctx->stream);
     rc = stage_redistancing_t<T>(ctx);
-    const int joined = join_elements(ctx);  // after an error too: read-back calls wait on the stream
+    const bool beside = ctx->el_beside;
+    if (rc && beside) cudaStreamSynchronize(ctx->el_stream);  // read-back calls find a finished build
+    const int joined = join_elements(ctx);
     if (rc || (rc = joined)) return rc;
     cudaEventRecord(ctx->ev[5], ctx->stream);
     CK(cudaEventSynchronize(ctx->ev[5]));
-    rc = check_err(ctx, "gg_step");
+    // No kernel after the redistancing's plan raises an error, so one that the plan's check did
+    // not see is the build's, and carries the name it has where the build ran before the plan.
+    rc = check_err(ctx, beside ? "redistancing plan" : "gg_step");
     if (rc) return rc;
     if (tuning) {  // device time per voxel-update of each stage under this candidate
         const double vox = (double)std::max(1LL, *ctx->h_total_vox);

@@ -87,3 +87,35 @@ def test_list_capacity_exhausted(gpu):
             gh.set_lists(off, ids)
         assert ei.value.code == gpu.GG_ERR_LIST_OVERFLOW
         assert f"has {max(lens)} entries" in str(ei.value)
+
+
+def test_element_build_overflow_is_named_whatever_it_runs_beside(gpu):
+    """A capacity of the element build runs out (one cube of 20^3 among 4^3 cubes: fewer than 256
+    neighbours, more than 256 distinct neighbour lists): the step fails with the same code and
+    text, the capacity named, whether the overflow happens before or after the redistancing's
+    plan is checked, and the read-back calls still answer."""
+    n, c = 36, 4
+    ax = np.arange(n) // c
+    cells = n // c
+    lab = 2 + ax[None, None, :] + cells * ax[None, :, None] + cells * cells * ax[:, None, None]
+    lab[8:28, 8:28, 8:28] = 1
+    _, lab = np.unique(lab, return_inverse=True)
+    lab = (1 + lab.reshape(n, n, n)).astype(np.uint32)
+    G = int(lab.max())
+    ms = msgen.Microstructure(labels=lab, euler=np.zeros((G, 3)), stored_energy=np.zeros(G), seeds=np.zeros((G, 3)))
+    ext, counts = ms.grain_extents()
+    texts = set()
+    for precision in (gpu.PRECISION_FP64, gpu.PRECISION_MIXED):
+        for _ in range(4):
+            with gpu.GrainHandler(n, 5, 0.2, G, precision=precision, correction=True, unique_energies=False,
+                                  mobility_model=True) as gh:
+                gh.load(lab, ext, counts)
+                gh.default_lists()
+                with pytest.raises(gpu.GGError) as ei:
+                    gh.step()
+                assert ei.value.code == gpu.GG_ERR_POOL_EXHAUSTED
+                texts.add(str(ei.value))
+                assert gh.stats().exists.shape == (G + 1,)
+                assert len(gh.neighbors(1)) <= 256
+    (text,) = texts
+    assert "redistancing plan: more than 256 distinct neighbour lists" in text
