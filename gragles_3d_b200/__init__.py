@@ -281,8 +281,9 @@ class GrainHandler:
         return self._check(load_library().gg_loop(self._h))
 
     def launch_config(self) -> tuple:
-        """(CTAs per SM of each stage's kernels, chosen): the stages are the convolution with
-        the correction, lists, comparison, level set and redistancing."""
+        """(CTAs per SM, chosen): of the correction, the list update, the comparison and the
+        marching cubes; the fifth entry (redistancing), and without the correction the first,
+        stays at the default (those kernels size their own grids)."""
         m = np.zeros(5, np.int32)
         done = self._check(load_library().gg_launch_config(self._h, _p(m)))
         return tuple(int(v) for v in m), bool(done)

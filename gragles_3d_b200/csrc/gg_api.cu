@@ -113,9 +113,10 @@ struct gg_ctx {
     // grid coarsening (grainhdl::gridCoarsement): ngrains at the last coarsening, and
     // NumberOfPointsPerGrain
     int coarse_ref = 0, points_per_grain = 0;
-    // launch configuration: CTAs per SM of each stage's grid-stride kernels (convolution
-    // with the correction, lists, comparison, level set, redistancing), chosen by the
-    // autotuner when it is on; the comparison launches a fixed multiple of its entry
+    // launch configuration: CTAs per SM of the correction, the list update, the comparison
+    // (which launches a fixed multiple of its entry) and the marching cubes, chosen by the
+    // autotuner when it is on.  The convolutions and the redistancing size their own grids, so
+    // without the correction nothing reads the first entry, and nothing reads the last.
     int mult[5] = {8, 8, 4, 8, 8};
     int tune_next = -1;         // candidate the next tuning step runs, -1: not tuning
     double tune_cost[5][8] = {};
@@ -127,14 +128,17 @@ struct gg_ctx {
 
 namespace {
 
-// The autotuner's candidates: CTAs per SM for the grid-stride stage kernels.  Every stage
-// kernel walks its tiles grid-stride and computes each grain's results inside one CTA, so
+// The autotuner's candidates: CTAs per SM for the grid-stride stage kernels.  Each of these
+// kernels walks its tiles grid-stride and computes each grain's results inside one CTA, so
 // the grid changes only the speed, never the results.
 constexpr int kTuneCand[] = {2, 4, 8, 16, 32};
 constexpr int kNumTune = 5;
 enum Stage { ST_CONV = 0, ST_LISTS, ST_COMPARE, ST_LEVELSET, ST_REDIST };
 
 int stage_grid(const gg_ctx* c, int s);
+
+// Whether a kernel of stage s launches by its entry of the launch configuration.
+bool tuned(const gg_ctx* c, int s) { return s == ST_CONV ? c->correction : s != ST_REDIST; }
 
 int fail(gg_ctx* c, int code, const char* fmt, ...) {
     char buf[512];
@@ -349,12 +353,12 @@ int redistance(gg_ctx* ctx, int in_a, int out_a, const int* toff, int side, bool
     r.err = ctx->d_err;
     if (classes) {  // per size class of the output boxes (their tiles from toff)
         launch_redist_classes(ctx->G, toff, ctx->d_box[out_a], ctx->d_toff_rcls, ctx->stream);
-        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, ctx->d_toff_rcls, &ctx->aux, ctx->stream);
+        launch_redistance<T>(r, 0, side, ctx->d_toff_rcls, &ctx->aux, ctx->stream);
         int nc = 0;
         for (int c = 0; c < kRedistClasses && (c == 0 || redist_side(c - 1) < side); c++) nc++;
         ctx->launches += 1 + 2 * nc;
     } else {
-        launch_redistance<T>(r, stage_grid(ctx, ST_REDIST), side, nullptr, nullptr, ctx->stream);
+        launch_redistance<T>(r, ctx->grid, side, nullptr, nullptr, ctx->stream);
         ctx->launches += 2;
     }
     CK(cudaGetLastError());
@@ -858,7 +862,8 @@ int step_t(gg_ctx* ctx, gg_step_stats* st) {
     // the autotuner: loops 1 .. kNumTune (loop 0 has no correction) each run one candidate
     const bool tuning = ctx->tune_next >= 0 && ctx->loop >= 1;
     if (tuning)
-        for (int s = 0; s < 5; s++) ctx->mult[s] = kTuneCand[ctx->tune_next];
+        for (int s = 0; s < 5; s++)
+            if (tuned(ctx, s)) ctx->mult[s] = kTuneCand[ctx->tune_next];
     cudaEventRecord(ctx->ev[0], ctx->stream);
     int rc = stage_convolution_t<T>(ctx);
     if (rc) return rc;
@@ -892,7 +897,7 @@ int step_t(gg_ctx* ctx, gg_step_stats* st) {
                 int best = 0;
                 for (int c = 1; c < kNumTune; c++)
                     if (ctx->tune_cost[s][c] < ctx->tune_cost[s][best]) best = c;
-                ctx->mult[s] = kTuneCand[best];
+                if (tuned(ctx, s)) ctx->mult[s] = kTuneCand[best];
             }
             ctx->tune_next = -1;
         }

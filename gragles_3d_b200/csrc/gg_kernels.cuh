@@ -429,8 +429,9 @@ __host__ __device__ constexpr int redist_units(int c) {
 }
 // class_toff: kRedistClasses tile tables of stride G + 2 (ceil(n / redist_units(c)) tiles
 // per grain of class c),
-// from launch_redist_classes; null: one launch over `a.toff` sized for `side`.  aux: the
-// context's own side streams, which wait for s and which s waits for (used with class_toff).
+// from launch_redist_classes; null: one launch over `a.toff` sized for `side`, of 2 grid CTAs (a
+// class's launches take their grid from what the device holds).  aux: the context's own side
+// streams, which wait for s and which s waits for (used with class_toff).
 constexpr int kSideStreams = 3;
 struct SideStreams {
     cudaStream_t stream[kSideStreams];

@@ -61,7 +61,7 @@ typedef struct {
                                    (int)(N / n_grains^(1/3) + 0.5), grainhdl.cpp:221) */
     double coarsening_gradient; /* GridCoarsementGradient (0 = 0.95, the Settings default) */
     int32_t autotune;           /* 1: loops 1..5 each time one launch configuration (2, 4, 8, 16 and 32
-                                   CTAs per SM for the grid-stride kernels of every stage) and the
+                                   CTAs per SM for the kernels gg_launch_config names) and the
                                    rest run each stage with its fastest; results do not depend on it */
 } gg_params;
 
@@ -125,11 +125,13 @@ int gg_step(gg_ctx* ctx, gg_step_stats* stats);
  * a grid coarsening). */
 int gg_domain_size(gg_ctx* ctx);
 
-/* The launch configuration in use: CTAs per SM of the grid-stride kernels of each stage
- * (convolution with the correction, lists, comparison, level set, redistancing; the
- * comparison's grid is up to 16 times its entry, a CTA a share of the tiles).  No
- * counterpart in the reference (its parallel loops are OpenMP over grains).  Returns 1
- * once the autotuner has chosen them (or when it is off), 0 while it is still trying. */
+/* The launch configuration in use: CTAs per SM of the correction, the list update, the
+ * comparison (its grid is up to 16 times its entry, a CTA a share of the tiles), the marching
+ * cubes, and a fifth entry for the redistancing.  The convolutions and the redistancing take
+ * their grids from what the device holds, so the autotuner leaves the fifth entry, and without
+ * the correction the first, at the default.  No counterpart in the reference (its parallel
+ * loops are OpenMP over grains).  Returns 1 once the autotuner has chosen them (or when it is
+ * off), 0 while it is still trying. */
 int gg_launch_config(gg_ctx* ctx, int32_t ctas_per_sm[5]);
 
 /* The stages of one iteration, for stage-level testing, in the order gg_step runs

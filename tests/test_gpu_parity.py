@@ -419,6 +419,31 @@ def test_autotuned_launches_give_the_same_bits(gpu, oracle):
         assert np.array_equal(ea, eb) and np.array_equal(va, vb) and np.array_equal(ba, bb)
 
 
+@pytest.mark.parametrize("correction", [False, True])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_autotuner_leaves_entries_alone_that_no_kernel_reads(gpu, precision, correction):
+    """The convolutions and the redistancing size their own grids: the autotuner reports the
+    default for the redistancing, and for the convolution's stage without the correction."""
+    N, G = 32, 60
+    ms = msgen.voronoi(N, G, seed=1032)
+    ext, counts = ms.grain_extents()
+    cfg = {}
+    for tune in (False, True):
+        with gpu.GrainHandler(N, 5, 0.2, G, precision=precision, autotune=tune, correction=correction,
+                              unique_energies=False, mobility_model=True) as gh:
+            gh.load(ms.labels, ext, counts)
+            gh.default_lists()
+            gh.set_orientations(ms.euler)
+            for _ in range(6):
+                gh.step()
+            cfg[tune], done = gh.launch_config()
+            assert done
+    assert cfg[True][4] == cfg[False][4]
+    if not correction:
+        assert cfg[True][0] == cfg[False][0]
+    assert all(c in (2, 4, 8, 16, 32) for c in cfg[True])
+
+
 def test_cpp_host_runs_the_reference_mode4_case(gpu, tmp_path):
     """The C++ host (gragles_3d_b200/gg_run, the reference's mode-4 main over the C ABI) reads
     the reference's own input files and parameters.xml and reproduces the compiled
