@@ -34,7 +34,7 @@ EXPORTED = [
     "gg_get_idlocal", "gg_grain_count", "gg_loop", "gg_convolve_boxes_f64", "gg_convolve_boxes_mixed",
     "gg_convolve_boxes_f64_noalloc", "gg_set_orientations", "gg_set_stored_energy", "gg_get_elements",
     "gg_voxel_container", "gg_get_faces", "gg_domain_size", "gg_rtree_lists", "gg_rtree_lists_from_boxes",
-    "gg_launch_config",
+    "gg_launch_config", "gg_set_work_split",
 ]
 
 
@@ -89,6 +89,7 @@ def load_library(path: str = LIB_PATH):
     L.gg_default_lists.argtypes = [vp]
     L.gg_rtree_lists.argtypes = [vp]
     L.gg_launch_config.argtypes = [vp, vp]
+    L.gg_set_work_split.argtypes = [vp, i32, i32]
     L.gg_rtree_lists_from_boxes.argtypes = [i32, vp, vp, vp, vp, i64]
     L.gg_rtree_lists_from_boxes.restype = i64
     L.gg_step.argtypes = [vp, C.POINTER(StepStats)]
@@ -287,6 +288,11 @@ class GrainHandler:
         m = np.zeros(5, np.int32)
         done = self._check(load_library().gg_launch_config(self._h, _p(m)))
         return tuple(int(v) for v in m), bool(done)
+
+    def set_work_split(self, correction_passes: int = 0, elements_beside: int = -1) -> None:
+        """How the correction's work items and the element build are split (see gg_set_work_split),
+        for tests and measurements; results do not depend on it."""
+        self._check(load_library().gg_set_work_split(self._h, correction_passes, elements_beside))
 
     @property
     def domain_size(self) -> int:

@@ -120,6 +120,9 @@ struct gg_ctx {
     int mult[5] = {8, 8, 4, 8, 8};
     int tune_next = -1;         // candidate the next tuning step runs, -1: not tuning
     double tune_cost[5][8] = {};
+    // gg_set_work_split: passes a work item of the correction, the element build beside the
+    // redistancing (0 / -1: by the rules)
+    int split_passes = 0, split_beside = -1;
     // element counts of the N-dependent tables' device buffers (reused when they fit)
     size_t tw_cap = 0, gt_cap = 0, circ_cap = 0, bmat_cap = 0;
     size_t tw_off_cap = 0, g_off_cap = 0, c_off_cap = 0, boff_cap = 0;
@@ -422,7 +425,8 @@ int correct_convolution(gg_ctx* ctx) {
     c.el = ctx->el;
     c.ph = physics(ctx);
     c.err = ctx->d_err;
-    c.item_vox = correction_item_voxels(*ctx->h_total_vox, ctx->num_sms);  // the last step's voxels
+    c.item_vox = ctx->split_passes ? ctx->split_passes * correction_pass_voxels()
+                                   : correction_item_voxels(*ctx->h_total_vox, ctx->num_sms);  // the last step's voxels
     launch_work_order(ctx->work, ctx->G, ctx->d_toff_one, ctx->d_box[p], c.item_vox, ctx->stream);
     c.order = ctx->work.order;
     c.item_off = ctx->work.item_off;
@@ -715,7 +719,8 @@ int level_set_t(gg_ctx* ctx, int p, int regrid) {
         // With more turns a warp both mostly take turns and disturb each other: 19.2 -> 19.9 ms
         // for 20,000.
         constexpr int kTurns = 12, kWarpsSM = 6;
-        const bool beside = ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
+        const bool beside = ctx->split_beside >= 0 ? ctx->split_beside
+                                                   : ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
         cudaStream_t t = beside ? ctx->el_stream : ctx->stream;
         if (beside) {
             CK(cudaEventRecord(ctx->el_fork, ctx->stream));
@@ -1422,6 +1427,13 @@ int gg_launch_config(gg_ctx* ctx, int32_t ctas_per_sm[5]) {
     if (!ctx || !ctas_per_sm) return GG_ERR_INVALID;
     for (int s = 0; s < 5; s++) ctas_per_sm[s] = ctx->mult[s];
     return ctx->tune_next >= 0 ? 0 : 1;
+}
+int gg_set_work_split(gg_ctx* ctx, int32_t correction_passes, int32_t elements_beside) {
+    if (!ctx || correction_passes < 0 || correction_passes > 1024 || elements_beside < -1 || elements_beside > 1)
+        return GG_ERR_INVALID;
+    ctx->split_passes = correction_passes;
+    ctx->split_beside = elements_beside;
+    return GG_OK;
 }
 int gg_loop(gg_ctx* ctx) { return ctx ? ctx->loop : GG_ERR_INVALID; }
 

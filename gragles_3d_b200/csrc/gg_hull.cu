@@ -1104,7 +1104,7 @@ __device__ __forceinline__ double sqdist3(double x, double y, double z, const do
 
 constexpr int kCThreads = 256;
 constexpr int kCVox = 4096;           // voxels of one pass: a run of the box in [z][y][x] order
-constexpr int kCItem = 4 * kCVox;     // voxels of one work item: a grain's box is cut into runs of these
+constexpr int kCItem = 4 * kCVox;     // voxels of a long work item (a short one: kCVox); a box is cut into such runs
 constexpr int kLV = 2;                // voxels per lane: a packet is 32 kLV voxels of one neighbour
 constexpr int kPacket = 32 * kLV;
 constexpr int kWarpTies = 8;          // near ties a packet settles voxel by voxel with the whole warp
@@ -1711,6 +1711,7 @@ __global__ void __launch_bounds__(kCThreads, 3) correction_kernel(const __grid_c
 }  // namespace
 
 size_t elements_scratch_per_cta() { return kElemScratch; }
+int correction_pass_voxels() { return kCVox; }
 int correction_item_voxels(long long total, int num_sms) {
     // A long run per item pays the staging once; below eight long runs per resident CTA (three
     // an SM) single passes spread the work better: 30 grains of 90^3 voxels, one of which is

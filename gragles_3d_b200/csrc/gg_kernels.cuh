@@ -324,8 +324,10 @@ struct CorrectionArgs {
     int item_vox;             // box voxels of an item
     int* err;
 };
-// Box voxels of one work item of the correction, for `total` voxels over all boxes.
+// Box voxels of one work item of the correction, for `total` voxels over all boxes: whole passes
+// of correction_pass_voxels().
 int correction_item_voxels(long long total, int num_sms);
+int correction_pass_voxels();
 template <typename T>
 void launch_correction(const CorrectionArgs<T>& a, int grid, cudaStream_t s);
 

@@ -134,6 +134,13 @@ int gg_domain_size(gg_ctx* ctx);
  * off), 0 while it is still trying. */
 int gg_launch_config(gg_ctx* ctx, int32_t ctas_per_sm[5]);
 
+/* How a context splits work that it otherwise splits by the size of its domain, for tests and
+ * measurements; results do not depend on it.  correction_passes: passes of 4,096 voxels in a
+ * work item of the correction (1 to 1024; 0, the default: 4 where the boxes are many, else 1).
+ * elements_beside: the element build on a stream of its own beside the redistancing (1), before
+ * it (0), or by the number of grains (-1, the default). */
+int gg_set_work_split(gg_ctx* ctx, int32_t correction_passes, int32_t elements_beside);
+
 /* The stages of one iteration, for stage-level testing, in the order gg_step runs
  * them.  Each stands in for the grainhdl method named. */
 int gg_stage_convolution(gg_ctx* ctx);       /* switchDistancebuffer + convolution, :839-849 */

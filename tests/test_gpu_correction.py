@@ -200,3 +200,56 @@ def test_correction_of_large_hulls_matches_oracle(gpu, oracle):
             assert bool(st.exists[i]) and inf["exists"], f"step {s} grain {i}"
             assert gh.elements(i) == osim.elements(i), f"step {s} grain {i}: elements"
             assert abs(st.volume[i] - inf["volume"]) <= 1e-9 * inf["volume"], f"step {s} grain {i}: volume"
+
+
+@pytest.mark.parametrize("grains", [60, 3])
+def test_work_split_gives_the_same_bits(gpu, oracle, grains):
+    """A work item of the correction of one pass (small domains) and of several (large ones), the
+    element build beside the redistancing (few grains) and before it (many): fields, elements
+    and statistics equal bit for bit on both precisions, and the FP64 path's elements, hull
+    neighbours and volumes are the oracle's.  Boxes of about 4 and of 38 passes."""
+    if grains == 60:
+        n, (ms, see) = N, _case()
+    else:
+        n, see = 44, np.array([3.0, 1.0, 2.0]) * 1e5 * 2.5e-10 * 2.52e-4
+        ms = msgen.voronoi(n, grains, seed=2144)
+        ms.euler[:] = np.array([[0.3, 0.5, 0.2], [0.38, 0.46, 0.25], [1.1, 0.9, 2.0]])
+    ext, counts = ms.grain_extents()
+    osim = None
+    for precision in (gpu.PRECISION_FP64, gpu.PRECISION_MIXED):
+        first = None
+        for split in ((1, 0), (4, 0), (4, 1), (3, 0), (1, 1), (0, -1)):
+            with gpu.GrainHandler(n, BORDER, 0.2, grains, precision=precision, correction=True, **PHYS) as gh:
+                gh.load(ms.labels, ext, counts)
+                gh.default_lists()
+                gh.set_orientations(ms.euler)
+                gh.set_stored_energy(see)
+                gh.set_work_split(*split)
+                if osim is None:
+                    lists = [gh.comparison_list(g) for g in range(1, grains + 1)]
+                    off = np.concatenate([[0, 0], np.cumsum([r.size for r in lists])]).astype(np.int64)
+                    osim = oracle.OracleSim(n, BORDER, 0.2, ms.labels, ext, counts,
+                                            lists=(off, np.concatenate(lists).astype(np.uint32)))
+                    osim.set_physics(True, unique_energies=False, mobility_model=True, triple_line_drag=20.0,
+                                     stored_energy=True)
+                    osim.set_orientations(ms.euler)
+                    osim.set_stored_energy(see)
+                    for _ in range(4):
+                        osim.step()
+                for _ in range(4):
+                    gh.step()
+                st = gh.stats()
+                alive = [g for g in range(1, grains + 1) if st.exists[g]]
+                got = [st.exists, st.volume, st.surface, st.boxes, st.n_neighbors]
+                got += [np.array(gh.elements(g)) for g in alive] + [gh.sdf(g)[1] for g in alive]
+                if first is None:
+                    first = got
+                assert all(np.array_equal(a, b) for a, b in zip(first, got)) and len(first) == len(got), split
+                if precision == gpu.PRECISION_FP64 and split[0] == 4:
+                    for g in range(1, grains + 1):
+                        inf = osim.info(g)
+                        assert bool(st.exists[g]) == inf["exists"], f"{split} grain {g}"
+                        if inf["exists"]:
+                            assert abs(st.volume[g] - inf["volume"]) <= 1e-9 * inf["volume"], f"{split} grain {g}"
+                            assert np.array_equal(gh.neighbors(g), osim.neighbors(g)), f"{split} grain {g}"
+                            assert gh.elements(g) == osim.elements(g), f"{split} grain {g}"

@@ -106,9 +106,10 @@ def test_element_build_overflow_is_named_whatever_it_runs_beside(gpu):
     ext, counts = ms.grain_extents()
     texts = set()
     for precision in (gpu.PRECISION_FP64, gpu.PRECISION_MIXED):
-        for _ in range(4):
+        for beside in (0, 1, -1, -1):
             with gpu.GrainHandler(n, 5, 0.2, G, precision=precision, correction=True, unique_energies=False,
                                   mobility_model=True) as gh:
+                gh.set_work_split(elements_beside=beside)
                 gh.load(lab, ext, counts)
                 gh.default_lists()
                 with pytest.raises(gpu.GGError) as ei:
