@@ -259,6 +259,36 @@ def test_contour_at_every_cta_size_bitexact(gpu, oracle, G):
             assert np.array_equal(gh.neighbors(g), osim.neighbors(g)), f"grain {g}"
 
 
+def test_redistancing_at_class_edges_bitexact(gpu, oracle):
+    """Output boxes at the edges of the redistancing's size classes beside each other in one step:
+    56 | 57 (two classes), 63 and 64 (the last bits of the 64-bit sign masks), 65 to 67 (runtime
+    pitch) and small ones; every field equals the oracle's bit for bit.  Eight slabs of 8
+    layers, each with one square grain and four in the rest."""
+    n, border = 64, 5
+    lab = np.zeros((n, n, n), np.int64)
+    G = 0
+    for k, a in enumerate((47, 48, 54, 55, 56, 57, 58, 30)):
+        for ys, xs in ((slice(0, a), slice(0, a)), (slice(0, 32), slice(a, n)), (slice(32, n), slice(a, n)),
+                       (slice(a, n), slice(0, a // 2)), (slice(a, n), slice(a // 2, a))):
+            G += 1
+            lab[8 * k:8 * k + 8, ys, xs] = G
+    ms = msgen.Microstructure(lab.astype(np.uint32), np.zeros((G, 3)), np.zeros(G), np.zeros((G, 3)))
+    ext, counts = ms.grain_extents()
+    gh = gpu.GrainHandler(n, border, 0.2, G, precision=0)
+    gh.load(ms.labels, ext, counts)
+    gh.default_lists()
+    osim = oracle.OracleSim(n, border, 0.2, ms.labels, ext, counts, lists=_default_lists_from(gh))
+    for s in range(3):
+        assert gh.step()["grain_count"] == osim.step()
+        st = gh.stats()
+        sides = set(int(b[1] - b[0]) for g, b in enumerate(st.boxes) if st.exists[g])
+        assert {33, 56, 57, 63, 64, 65, 66, 67} <= sides
+        for g in range(1, G + 1):
+            inf = osim.info(g)
+            assert bool(st.exists[g]) == inf["exists"] and tuple(st.boxes[g]) == inf["box"], f"step {s} grain {g}"
+            assert np.array_equal(osim.sdf(g)[1], gh.sdf(g)[1]), f"step {s} grain {g}: field"
+
+
 def test_loop_mixed_volume_tolerance(gpu, oracle):
     c, gh, osim = _pair(gpu, oracle, "border10", precision=1)
     worst = 0.0
