@@ -971,7 +971,7 @@ int supported_side(bool fp64) {
     int n = 8;
     for (;;) {
         const int m = n + 1;
-        bool ok = redist_smem_bytes(m, fp64) <= lim && mc_slab_bytes(m) + 40 * 1024 <= lim;
+        bool ok = redist_smem_bytes(m, fp64) <= lim && mc_slab_bytes(m) + kMcStaticBytes <= lim;
         if (fp64) ok = ok && m <= kConvF64MaxSide;
         else ok = ok && 3 * (size_t)m * (m | 1) * 4 <= lim;
         if (!ok || m > 4096) return n;

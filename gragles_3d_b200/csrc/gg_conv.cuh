@@ -22,8 +22,8 @@ struct ConvArgs {
     const long long* g_off;
 };
 
-// Largest box side the FP64 convolution takes (a plane and two complex half-spectra of it
-// fill 227 KB of shared memory).
+// Largest box side the FP64 convolution takes: a chosen bound, up to which it is tested.  (The
+// passes hold lines, not planes: at most 39 KB a warp at this side.)
 constexpr int kConvF64MaxSide = 97;
 // Five launches; nmax: the largest side among the boxes of the tiles.
 void launch_conv_f64(const ConvArgs& a, int nmax, cudaStream_t s);

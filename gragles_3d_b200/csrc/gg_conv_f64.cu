@@ -416,10 +416,15 @@ __global__ void __launch_bounds__(kThreads, 2) conv_x_inverse(ConvArgs a, int wa
 // Shared memory of a warp of each pass, in bytes, at side n: its twiddles and its lines (and
 // z's products, above kColChunk fragments).
 constexpr int kSlack = 16 * 8;
-int x_forward_bytes(int n) { return 16 * n + 8 * 8 * kRowFrags * pitch4(n) + kSlack; }
-int y_bytes(int n) { return 16 * n * (1 + kLP) + kSlack; }
-int z_bytes(int n) { return 16 * n * (1 + kLP * ((n + 7) / 8 > kColChunk ? 2 : 1)) + kSlack; }
-int x_inverse_bytes(int n) { return 16 * n + 16 * 8 * kRowFrags * pitch2(n / 2 + 1) + kSlack; }
+constexpr int kMaxSmem = 227 * 1024;
+constexpr int x_forward_bytes(int n) { return 16 * n + 8 * 8 * kRowFrags * pitch4(n) + kSlack; }
+constexpr int y_bytes(int n) { return 16 * n * (1 + kLP) + kSlack; }
+constexpr int z_bytes(int n) { return 16 * n * (1 + kLP * ((n + 7) / 8 > kColChunk ? 2 : 1)) + kSlack; }
+constexpr int x_inverse_bytes(int n) { return 16 * n + 16 * 8 * kRowFrags * pitch2(n / 2 + 1) + kSlack; }
+
+static_assert(x_forward_bytes(kConvF64MaxSide) <= kMaxSmem && y_bytes(kConvF64MaxSide) <= kMaxSmem &&
+                  z_bytes(kConvF64MaxSide) <= kMaxSmem && x_inverse_bytes(kConvF64MaxSide) <= kMaxSmem,
+              "a warp's buffers fit a CTA at the largest side");
 
 // CTAs of as many warps as fit (8 at most), whole waves of the CTAs that fit the device at once:
 // one wave for a few boxes, where every wave pays its start (0.100 -> 0.082 ms for 20 grains of
@@ -427,7 +432,6 @@ int x_inverse_bytes(int n) { return 16 * n + 16 * 8 * kRowFrags * pitch2(n / 2 +
 // for 2,000 of 128^3 against one).
 template <typename K>
 void launch_pass(K kernel, const ConvArgs& a, int warp_bytes, int nmax, cudaStream_t s) {
-    constexpr int kMaxSmem = 227 * 1024;
     const int warps = std::min(kMaxSmem / warp_bytes, kWarps);
     const size_t smem = (size_t)warps * warp_bytes;
     int dev = 0, sms = 148, per_sm = 0;

@@ -48,7 +48,7 @@ namespace {
 
 constexpr int kThreads = 384;
 constexpr int kR = 8;        // output rows per thread
-constexpr int kMaxNB = 5;    // 32-wide column groups of the largest side (138)
+constexpr int kMaxNB = 5;    // 32-wide column groups of the largest side (139)
 
 // Pitch of the shared-memory matrices: even, for the two-element reads, and 2 modulo 4, so that
 // the 32 lanes that read one column of 32 rows fall on 16 banks.

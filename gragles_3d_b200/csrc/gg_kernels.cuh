@@ -361,7 +361,9 @@ struct MCArgs {
 };
 template <typename T>
 void launch_mc(const MCArgs<T>& a, int grid, int side, int grains, int num_sms, cudaStream_t s);
-// Dynamic shared memory of the marching-cubes kernel for boxes up to `side`.
+// Static shared memory of the marching-cubes kernel, at most, at any CTA size, and its dynamic
+// shared memory for boxes up to `side`.
+constexpr size_t kMcStaticBytes = 48 * 1024;
 size_t mc_slab_bytes(int side);
 
 // ---- grid coarsening (gg_coarsen.cu) ----

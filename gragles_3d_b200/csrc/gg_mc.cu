@@ -107,6 +107,8 @@ __device__ __forceinline__ void hash_insert(unsigned* hkey, unsigned* hval, unsi
 template <typename T, int kThreads>
 __global__ void __launch_bounds__(kThreads, 768 / kThreads) mc_kernel(MCArgs<T> a, int slab_bytes) {
     static_assert(kThreads * 5 * sizeof(double) >= 2 * kHash * sizeof(unsigned), "ID collection aliases the volume buffer");
+    static_assert(2 * kThreads * 5 * sizeof(double) + 2 * kHash * sizeof(unsigned) + 256 * 10 + 256 <= kMcStaticBytes,
+                  "the arrays below fit the bound that the supported side is worked out with");
     __shared__ double vbuf[kThreads * 5];
     __shared__ double abuf[kThreads * 5];
     __shared__ int warp_sums[33];

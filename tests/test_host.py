@@ -2,6 +2,7 @@
 include/gg_b200.h declares (no compute calls without a GPU), the microstructure
 generator and its mode-4 files, and the replica aggregation of the multi-GPU
 bench path over a two-rank gloo group."""
+import ctypes
 import os
 import re
 import socket
@@ -48,6 +49,18 @@ def test_create_rejects_bad_parameters_without_touching_the_device():
     with pytest.raises(gg.GGError) as e:
         gg.GrainHandler(64, 10, 0.2, 5, precision=7)
     assert e.value.code == gg.GG_ERR_INVALID
+
+
+@pytest.mark.parametrize("name,side", [("gg_convolve_boxes_f64", 98), ("gg_convolve_boxes_mixed", 140)])
+def test_convolution_refuses_sides_above_its_bound(name, side):
+    """One past the largest side (97 FP64, 139 mixed), beside a small one, is refused before the
+    device is touched."""
+    import gragles_3d_b200 as gg
+
+    host = np.zeros(64)  # stands in for device memory: never read
+    sides, offs = np.array([4, side], np.int32), np.array([0, 64], np.int64)
+    p = lambda a: a.ctypes.data_as(ctypes.c_void_p)  # noqa: E731
+    assert getattr(gg.load_library(), name)(p(host), p(host), p(sides), p(offs), 2, 100, 0.2) == gg.GG_ERR_UNSUPPORTED
 
 
 def test_generator_is_deterministic_and_consistent():
