@@ -1010,12 +1010,22 @@ void free_all(gg_ctx* c) {
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
-}  // namespace
+// Runs f, which makes host tables, and turns what it throws into a status code: nothing is thrown
+// across the C ABI.  The context is the one that f works on, null until there is one.
+template <typename F>
+int guarded(gg_ctx* const& ctx, F&& f) {
+    try {
+        return f();
+    } catch (...) {
+        try {
+            return fail(ctx, GG_ERR_POOL_EXHAUSTED, "out of host memory");
+        } catch (...) {
+            return GG_ERR_POOL_EXHAUSTED;
+        }
+    }
+}
 
-extern "C" {
-
-int gg_create(const gg_params* params, gg_ctx** out) {
-    gg_ctx* ctx = nullptr;
+int create(const gg_params* params, gg_ctx** out, gg_ctx*& ctx) {
     if (!params || !out) return GG_ERR_INVALID;
     *out = nullptr;
     ctx = new gg_ctx();
@@ -1152,6 +1162,15 @@ int gg_create(const gg_params* params, gg_ctx** out) {
         CK(cudaMemset(ctx->d_idoff[a], 0, sizeof(long long) * G1));
     }
     return upload_tables(ctx);
+}
+
+}  // namespace
+
+extern "C" {
+
+int gg_create(const gg_params* params, gg_ctx** out) {
+    gg_ctx* ctx = nullptr;
+    return guarded(ctx, [&] { return create(params, out, ctx); });
 }
 
 int gg_destroy(gg_ctx* ctx) {
@@ -1316,7 +1335,8 @@ int gg_rtree_lists(gg_ctx* ctx) {
 
 int gg_stage_convolution(gg_ctx* ctx) {
     if (!ctx || !ctx->loaded) return GG_ERR_INVALID;
-    int rc = ctx->fp64 ? stage_convolution_t<double>(ctx) : stage_convolution_t<float>(ctx);
+    // a grid coarsening makes its tables
+    int rc = guarded(ctx, [&] { return ctx->fp64 ? stage_convolution_t<double>(ctx) : stage_convolution_t<float>(ctx); });
     return rc ? rc : check_err(ctx, "convolution");
 }
 int gg_stage_update_lists(gg_ctx* ctx) {
@@ -1346,7 +1366,7 @@ int gg_stage_redistancing(gg_ctx* ctx) {
 
 int gg_step(gg_ctx* ctx, gg_step_stats* stats) {
     if (!ctx || !ctx->loaded) return GG_ERR_INVALID;
-    return ctx->fp64 ? step_t<double>(ctx, stats) : step_t<float>(ctx, stats);
+    return guarded(ctx, [&] { return ctx->fp64 ? step_t<double>(ctx, stats) : step_t<float>(ctx, stats); });
 }
 
 int gg_get_grain_stats(gg_ctx* ctx, uint8_t* exists, double* volume, double* surface, int32_t* boxes,
@@ -1527,8 +1547,12 @@ int gg_get_elements(gg_ctx* ctx, int32_t id, int32_t counts[4]) {
     return GG_OK;
 }
 
-int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* sides, const int64_t* offs,
-                          int32_t n_boxes, int32_t domain_size, double time_step) {
+}  // extern "C"
+
+namespace {
+
+int convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* sides, const int64_t* offs,
+                       int32_t n_boxes, int32_t domain_size, double time_step) {
     gg_ctx* ctx = nullptr;  // for CK: no context to carry a message
     if (!d_in || !d_out || !sides || !offs || n_boxes < 1 || domain_size < 1) return GG_ERR_INVALID;
     int nmax = 0;
@@ -1604,8 +1628,8 @@ int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* side
     return GG_OK;
 }
 
-int gg_convolve_boxes_mixed(const float* d_in, float* d_out, const int32_t* sides, const int64_t* offs,
-                            int32_t n_boxes, int32_t domain_size, double time_step) {
+int convolve_boxes_mixed(const float* d_in, float* d_out, const int32_t* sides, const int64_t* offs,
+                         int32_t n_boxes, int32_t domain_size, double time_step) {
     gg_ctx* ctx = nullptr;  // for CK: no context to carry a message
     if (!d_in || !d_out || !sides || !offs || n_boxes < 1 || domain_size < 1) return GG_ERR_INVALID;
     int nmax = 0;
@@ -1699,6 +1723,26 @@ int gg_convolve_boxes_mixed(const float* d_in, float* d_out, const int32_t* side
     if (e & ERR_TIMEOUT) return GG_ERR_CUDA;
     if (e) return GG_ERR_UNSUPPORTED;
     return GG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int gg_convolve_boxes_f64(const double* d_in, double* d_out, const int32_t* sides, const int64_t* offs,
+                          int32_t n_boxes, int32_t domain_size, double time_step) {
+    gg_ctx* const ctx = nullptr;
+    return guarded(ctx, [&] {
+        return convolve_boxes_f64(d_in, d_out, sides, offs, n_boxes, domain_size, time_step);
+    });
+}
+
+int gg_convolve_boxes_mixed(const float* d_in, float* d_out, const int32_t* sides, const int64_t* offs,
+                            int32_t n_boxes, int32_t domain_size, double time_step) {
+    gg_ctx* const ctx = nullptr;
+    return guarded(ctx, [&] {
+        return convolve_boxes_mixed(d_in, d_out, sides, offs, n_boxes, domain_size, time_step);
+    });
 }
 
 }  // extern "C"

@@ -29,7 +29,7 @@ extern "C" {
 #define GG_OK 0
 #define GG_ERR_INVALID (-1)          /* bad argument or call order */
 #define GG_ERR_CUDA (-2)             /* a CUDA call failed */
-#define GG_ERR_POOL_EXHAUSTED (-3)   /* box pool or scratch capacity exceeded */
+#define GG_ERR_POOL_EXHAUSTED (-3)   /* box pool, scratch or host memory exceeded */
 #define GG_ERR_LIST_OVERFLOW (-4)    /* a comparison or neighbour list exceeded its capacity */
 #define GG_ERR_UNSUPPORTED (-5)      /* option not implemented on this path */
 

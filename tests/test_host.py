@@ -63,6 +63,33 @@ def test_convolution_refuses_sides_above_its_bound(name, side):
     assert getattr(gg.load_library(), name)(p(host), p(host), p(sides), p(offs), 2, 100, 0.2) == gg.GG_ERR_UNSUPPORTED
 
 
+@pytest.mark.parametrize("name", ["gg_convolve_boxes_f64", "gg_convolve_boxes_mixed"])
+def test_out_of_host_memory_is_a_status_code(name):
+    """Host tables that do not fit the address space (a child process with a limit on its own):
+    the C entry returns a status, it does not throw or abort."""
+    import subprocess
+    import sys
+
+    import gragles_3d_b200 as gg
+
+    child = """
+import ctypes, resource, sys
+import numpy as np
+lib = ctypes.CDLL(sys.argv[1])
+n = 2_000_000
+sides, offs, host = np.ones(n, np.int32), np.arange(n, dtype=np.int64) * 4, np.zeros(64)
+p = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+f = getattr(lib, sys.argv[2])
+f.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 2 + [ctypes.c_double]
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (used + (24 << 20),) * 2)
+print(f(p(host), p(host), p(sides), p(offs), n, 100, 0.2))
+"""
+    run = subprocess.run([sys.executable, "-c", child, gg.LIB_PATH, name], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr
+    assert int(run.stdout) == gg.GG_ERR_POOL_EXHAUSTED
+
+
 def test_generator_is_deterministic_and_consistent():
     from gragles_3d_b200 import microstructure as msgen
 
