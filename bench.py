@@ -506,8 +506,8 @@ def main():
 
     st_m, st_d = stage_means(reps_m), stage_means(reps_d)
     peak, peak_kind = read_peaks()
-    # the dominant kernel (the largest share of the launch list): the comparison,
-    # timed alone by the library's events on its stream
+    # the comparison, timed alone by the library's events on its stream (the second largest share
+    # of the launch list; the correction, the largest, works from shared-memory tables)
     ms_k = float(np.mean([r["ms_compare_kernel"] for r in reps_m]))
     vox_k = float(np.mean([r["compare_voxels"] for r in reps_m]))
     bytes_per = STAGE_BYTES["mixed"]["ms_comparison"]

@@ -716,8 +716,8 @@ int level_set_t(gg_ctx* ctx, int p, int regrid) {
         // a grain) leave most of the device idle at its end or throughout, runs beside it on a
         // stream of its own: level set and redistancing 7.7 -> 6.6 ms for 30 grains of 90^3 (4.7
         // since the build's loads run ahead), 3.15 -> 2.97 for 1,900, 12.6 -> 12.4 for 8,400.
-        // With more turns a warp both mostly take turns and disturb each other: 19.2 -> 19.9 ms
-        // for 20,000.
+        // The line lies where it was when 20,000 still lost by it (19.2 -> 19.9 ms); with the
+        // loads ahead they would not (17.69 -> 17.59).
         constexpr int kTurns = 12, kWarpsSM = 6;
         const bool beside = ctx->split_beside >= 0 ? ctx->split_beside
                                                    : ctx->grain_count <= kTurns * kWarpsSM * ctx->num_sms;
